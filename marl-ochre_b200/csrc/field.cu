@@ -339,6 +339,9 @@ __device__ __forceinline__ void diffuse_tile(const CUtensorMap* tm_src, const CU
         m1 = mask_of(1)[mi] != 0;
         walls = walls_of(1);
     }
+    // Step 1 issues plane STAGES into the stage that holds plane 0: every warp
+    // has to have read its plane-0 voxels by then.
+    __syncthreads();
 
     // One centre plane p: B = below, C = centre, A receives the plane above.
     auto step = [&](Vox& B, Vox& C, Vox& A, bool& mB, bool& mC, bool& mA, int p) -> bool {
