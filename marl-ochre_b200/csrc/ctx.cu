@@ -10,6 +10,7 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <new>
 #include <string>
 #include <vector>
@@ -19,6 +20,7 @@
 #include "ctx_impl.h"
 #include "surrogate.h"
 #include "internal.h"
+#include "kernel_setup.h"
 
 using namespace marl;
 
@@ -52,12 +54,53 @@ marl_status check_device(int* dev, int* sms) {
     cudaError_t e = cudaGetDeviceCount(&count);
     if (e != cudaSuccess || count == 0) return fail(MARL_ERR_NO_DEVICE, "no CUDA device (%s)", cudaGetErrorString(e));
     CK(cudaGetDevice(dev));
-    cudaDeviceProp prop;
-    CK(cudaGetDeviceProperties(&prop, *dev));
-    if (prop.major != 10) return fail(MARL_ERR_NO_DEVICE, "device %s is sm_%d%d; this library is built for sm_100a",
-                                      prop.name, prop.major, prop.minor);
-    *sms = prop.multiProcessorCount;
+    // Two attributes instead of cudaGetDeviceProperties, which takes 4 ms a
+    // call on the B200 host and was most of a small diffusion tick.
+    int major = 0;
+    CK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, *dev));
+    if (major != 10) {
+        cudaDeviceProp prop;
+        CK(cudaGetDeviceProperties(&prop, *dev));
+        return fail(MARL_ERR_NO_DEVICE, "device %s is sm_%d%d; this library is built for sm_100a", prop.name,
+                    prop.major, prop.minor);
+    }
+    CK(cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, *dev));
     return MARL_OK;
+}
+
+// Workspaces of the calls on caller-owned device buffers, stream-ordered from
+// a memory pool of the library's own.  The device's default pool gives its
+// memory back at every synchronisation (which each of these calls ends with),
+// so an allocation there cost 0.4 ms a call (up to 17 ms among other calls).
+// This pool keeps at most kWorkKeep bytes per device (a pool grows by 32 MiB,
+// so less would keep nothing) and returns what is beyond that at the next
+// synchronisation: 2 us a call.  Pools are safe with several host threads and
+// streams.
+constexpr uint64_t kWorkKeep = 32u << 20;
+
+static cudaError_t work_alloc(uint8_t** p, size_t bytes, int dev, cudaStream_t s) {
+    static std::mutex lock;
+    static cudaMemPool_t pools[kSetupDevices] = {};
+    if (dev >= 0 && dev < kSetupDevices) {
+        cudaMemPool_t pool = nullptr;
+        {
+            std::lock_guard<std::mutex> hold(lock);
+            if (!pools[dev]) {
+                cudaMemPoolProps props = {};
+                props.allocType = cudaMemAllocationTypePinned;
+                props.location.type = cudaMemLocationTypeDevice;
+                props.location.id = dev;
+                uint64_t keep = kWorkKeep;
+                if (cudaMemPoolCreate(&pool, &props) == cudaSuccess &&
+                    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+                    pools[dev] = pool;
+            }
+            pool = pools[dev];
+        }
+        if (pool && cudaMallocFromPoolAsync((void**)p, bytes, pool, s) == cudaSuccess) return cudaSuccess;
+        cudaGetLastError();
+    }
+    return cudaMallocAsync((void**)p, bytes, s);
 }
 
 void derive_consts(const marl_sim_params& p, FieldConsts* fk, CellConsts* ck) {
@@ -967,28 +1010,37 @@ marl_status marl_diffuse_device(float* field_dev, float* scratch_dev, const uint
     FieldConsts fk;
     CellConsts ck;
     derive_consts(*sim, &fk, &ck);
-    uint8_t* mask = nullptr;
-    uint32_t* err = nullptr;
-    CK(cudaMallocAsync((void**)&mask, (size_t)gz * gy * mask_pitch(gx), s));
-    CK(cudaMallocAsync((void**)&err, 4, s));
-    CK(cudaMemsetAsync(err, 0, 4, s));
-    CK(launch_repack_mask(occ_dev, mask, g, s));
-    DiffusionPlan plan;
-    if (!plan_diffusion(&plan, field_dev, scratch_dev, mask, g, 0, 16)) {
-        cudaFreeAsync(mask, s);
-        cudaFreeAsync(err, s);
-        return fail(MARL_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+    // Workspace: the error word, then the padded mask where the caller's rows
+    // cannot be read in place.
+    const bool in_place = mask_in_place(occ_dev, g);
+    uint8_t* work = nullptr;
+    CK(work_alloc(&work, 256 + (in_place ? 0 : (size_t)gz * gy * mask_pitch(gx)), dev, s));
+    uint32_t* err = reinterpret_cast<uint32_t*>(work);
+    cudaError_t e = cudaMemsetAsync(err, 0, 4, s);
+    const uint8_t* mask = occ_dev;
+    if (!in_place) {
+        mask = work + 256;
+        if (e == cudaSuccess) e = launch_repack_mask(occ_dev, work + 256, g, s);
     }
+    auto bail = [&](marl_status st) {
+        cudaFreeAsync(work, s);
+        return st;
+    };
+    if (e != cudaSuccess) return bail(cuda_fail(e, "occupancy mask"));
+    DiffusionPlan plan;
+    if (!plan_diffusion(&plan, field_dev, scratch_dev, mask, g, 0, 16))
+        return bail(fail(MARL_ERR_CUDA, "cuTensorMapEncodeTiled failed"));
     int cur = 0;  // 0: field_dev holds the live state, 1: scratch_dev does
-    for (uint32_t i = 0; i < substeps; ++i) {
-        CK(launch_diffuse(plan, cur, g, fk, 0, nullptr, err, s));
+    for (uint32_t i = 0; i < substeps && e == cudaSuccess; ++i) {
+        e = launch_diffuse(plan, cur, g, fk, 0, nullptr, err, s);
         cur ^= 1;
     }
-    if (cur != 0) CK(cudaMemcpyAsync(field_dev, scratch_dev, g.V() * 48, cudaMemcpyDeviceToDevice, s));
+    if (cur != 0 && e == cudaSuccess)
+        e = cudaMemcpyAsync(field_dev, scratch_dev, g.V() * 48, cudaMemcpyDeviceToDevice, s);
     uint32_t h_err = 0;
-    CK(cudaMemcpyAsync(&h_err, err, 4, cudaMemcpyDeviceToHost, s));
-    CK(cudaFreeAsync(mask, s));
-    CK(cudaFreeAsync(err, s));
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h_err, err, 4, cudaMemcpyDeviceToHost, s);
+    if (e != cudaSuccess) return bail(cuda_fail(e, "diffusion substeps"));
+    CK(cudaFreeAsync(work, s));
     CK(cudaStreamSynchronize(s));
     if (h_err) return fail(MARL_ERR_TIMEOUT, "device wait gave up (error bits 0x%x)", h_err);
     return MARL_OK;

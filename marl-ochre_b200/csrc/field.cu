@@ -755,6 +755,21 @@ cudaError_t launch_repack_mask(const uint8_t* occ, uint8_t* mask, const Grid& g,
     return cudaGetLastError();
 }
 
+// Whether the diffusion kernel can read the caller's dense occupancy as it
+// lies: rows of a multiple of 16 bytes at a 16-byte aligned address (the TMA
+// rules) in this device's own memory.  The kernel tests the bytes against zero,
+// so they need no normalising either.
+bool mask_in_place(const uint8_t* occ, const Grid& g) {
+    if (g.X % 16 || ((uintptr_t)occ & 15)) return false;
+    int dev = 0;
+    cudaPointerAttributes a;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaPointerGetAttributes(&a, occ) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == dev;
+}
+
 cudaError_t launch_unpack_mask(const uint8_t* mask, uint8_t* occ, const Grid& g, cudaStream_t s) {
     const size_t n = g.V();
     k_unpack_mask<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(mask, occ, g);

@@ -40,6 +40,7 @@ cudaError_t launch_light(const float* c4, const float* f, const uint8_t* mask, f
 cudaError_t launch_mass(const float* f, const Grid& g, double* partial, double* out, cudaStream_t s);
 size_t mass_partial_doubles();
 cudaError_t launch_repack_mask(const uint8_t* occ, uint8_t* mask, const Grid& g, cudaStream_t s);
+bool mask_in_place(const uint8_t* occ, const Grid& g);
 cudaError_t launch_unpack_mask(const uint8_t* mask, uint8_t* occ, const Grid& g, cudaStream_t s);
 
 // ---- cells ----

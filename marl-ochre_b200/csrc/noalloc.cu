@@ -7,8 +7,8 @@
 // framework's caching allocator or a fixed pool it may not grow), and
 // latency-critical loops where a cudaMalloc/cudaFree, and the device-wide
 // synchronisation it can imply, is not acceptable.  marl_diffuse_device
-// allocates a pitched occupancy mask and an error word on every call; this
-// variant allocates nothing.
+// allocates its error word, and a pitched occupancy mask where one is needed,
+// on every call; this variant allocates nothing.
 //
 // Scratch: one array, g_noalloc_scratch, holding (1) the ping-pong copy of the
 // field, (2) the occupancy mask with rows padded to 16 bytes (the TMA stride
@@ -24,9 +24,9 @@
 // loaded again at a new address).  The first call on a device also loads the
 // module, which reserves the array; that first call should come before any
 // stream capture.  All calls share the array and it keeps the last call's
-// contents: the mask is rewritten and the error word cleared at the start of
-// every call, and the scratch field is fully written by the first substep
-// before it is read.  Calls that overlap on the GPU (for example on two
+// contents: the mask is rewritten (unless the caller's rows are read in place)
+// and the error word cleared at the start of every call, and the scratch field
+// is fully written by the first substep before it is read.  Calls that overlap on the GPU (for example on two
 // streams at once) race on the array and must not be issued.
 #include <cuda_runtime.h>
 
@@ -94,9 +94,11 @@ extern "C" marl_status marl_diffuse_device_noalloc(float* field_dev, const uint8
     derive_consts(*sim, &fk, &ck);
     cudaError_t e = cudaMemsetAsync(err, 0, 4, s);
     if (e != cudaSuccess) return cuda_fail(e, "clear error word");
-    if ((e = launch_repack_mask(occupancy_dev, mask, g, s)) != cudaSuccess) return cuda_fail(e, "repack occupancy");
+    const bool in_place = mask_in_place(occupancy_dev, g);
+    if (!in_place && (e = launch_repack_mask(occupancy_dev, mask, g, s)) != cudaSuccess)
+        return cuda_fail(e, "repack occupancy");
     DiffusionPlan plan;
-    if (!plan_diffusion(&plan, field_dev, scratch, mask, g, 0, 16))
+    if (!plan_diffusion(&plan, field_dev, scratch, in_place ? occupancy_dev : mask, g, 0, 16))
         return fail(MARL_ERR_CUDA, "cuTensorMapEncodeTiled failed");
     int cur = 0;  // 0: field_dev holds the live state, 1: the scratch copy does
     for (uint32_t i = 0; i < substeps; ++i) {
