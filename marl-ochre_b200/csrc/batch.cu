@@ -405,9 +405,11 @@ int surrogate_cell_mode(const marl_batch* b) {
 // b->cur flipped by the number of substeps.
 marl_status enqueue_device_tick(marl_batch* b, cudaStream_t s, int cur) {
     const int n_runs = (int)b->runs.size();
+    const uint32_t split = surrogate_cell_mode(b) == kModePlain ? cell_quad_limit(b->num_sms) : 0;
+    const bool schedule = b->packed_cap > split;  // else the four-lane loop computes every schedule
     CK(cudaMemcpyAsync(b->d_runs, b->h_runs, (size_t)n_runs * sizeof(RunDesc), cudaMemcpyHostToDevice, s));
     CK(cudaMemsetAsync(&b->d_scalars()->ticket, 0, 4, s));
-    CK(launch_cell_schedule_batch(b->d_runs, n_runs, b->num_sms, s));
+    if (schedule) CK(launch_cell_schedule_batch(b->d_runs, n_runs, split, b->num_sms, s));
     const uint32_t S = b->sim.diffusion_substeps;
     uint32_t* err = &b->d_scalars()->err;
     if (S == 0) {
@@ -429,7 +431,7 @@ marl_status enqueue_device_tick(marl_batch* b, cudaStream_t s, int cur) {
                                          b->surr_pred, b->surr_rows, s);
         if (st) return st;
     }
-    CK(launch_cell_tick_batch(b->d_runs, n_runs, b->d_scalars(), b->ck, cur, b->num_sms, mode, s));
+    CK(launch_cell_tick_batch(b->d_runs, n_runs, b->d_scalars(), b->ck, cur, b->num_sms, mode, b->packed_cap, s));
     if (mode != kModePlain && total > 0)
         CK(launch_surrogate_count(b->surr_status, b->surr_err, total, b->surr_counters,
                                   reinterpret_cast<uint32_t*>(b->surr_counters + 4), s));
@@ -441,7 +443,8 @@ marl_status enqueue_device_tick(marl_batch* b, cudaStream_t s, int cur) {
 
 uint64_t device_tick_launches(const marl_batch* b) {
     const uint32_t S = b->sim.diffusion_substeps;
-    return 1 + (S ? S : b->runs.size()) + 4 + (b->surr ? 5 : 0);
+    const int either = !b->surr && b->packed_cap > cell_quad_limit(b->num_sms) ? 2 : 0;  // schedule, second loop
+    return (b->surr ? 1 : either) + (S ? S : b->runs.size()) + 4 + (b->surr ? 5 : 0);
 }
 
 marl_status launch_tick(marl_batch* b) {
@@ -553,9 +556,11 @@ marl_status apply_edits(marl_batch* b) {
 // host; ends with b->cur flipped by the number of substeps.
 marl_status enqueue_device_fate_tick(marl_batch* b, cudaStream_t s, int cur) {
     const int n_runs = (int)b->runs.size();
+    const uint32_t split = cell_quad_limit(b->num_sms);
+    const bool schedule = b->packed_cap > split;  // else the four-lane loop computes every schedule
     CK(launch_batch_population(b->d_runs, n_runs, b->d_fate_runs, s));
     CK(cudaMemsetAsync(&b->d_scalars()->ticket, 0, 4, s));
-    CK(launch_cell_schedule_batch(b->d_runs, n_runs, b->num_sms, s));
+    if (schedule) CK(launch_cell_schedule_batch(b->d_runs, n_runs, split, b->num_sms, s));
     const uint32_t S = b->sim.diffusion_substeps;
     uint32_t* err = &b->d_scalars()->err;
     if (S == 0) {
@@ -567,14 +572,15 @@ marl_status enqueue_device_fate_tick(marl_batch* b, cudaStream_t s, int cur) {
         cur ^= 1;
     }
     CK(launch_light_batch(b->d_runs, b->d_light_items, b->n_light_items, b->fk, cur, S > 0 ? 1 : 0, s));
-    CK(launch_cell_tick_batch(b->d_runs, n_runs, b->d_scalars(), b->ck, cur, b->num_sms, kModePlain, s));
+    CK(launch_cell_tick_batch(b->d_runs, n_runs, b->d_scalars(), b->ck, cur, b->num_sms, kModePlain, b->packed_cap, s));
     CK(launch_fate(b->d_fate_runs, n_runs, b->max_cap, err, b->sim, b->num_sms, s));
     return MARL_OK;
 }
 
 uint64_t device_fate_tick_launches(const marl_batch* b) {
     const uint32_t S = b->sim.diffusion_substeps;
-    return 1 + 1 + (S ? S : b->runs.size()) + 1 + 1 + 5;
+    const int either = b->packed_cap > cell_quad_limit(b->num_sms) ? 2 : 0;  // schedule, second loop
+    return 1 + either + (S ? S : b->runs.size()) + 1 + 1 + 5;
 }
 
 marl_status launch_device_fate_tick(marl_batch* b) {

@@ -295,17 +295,21 @@ marl_status enqueue_cell_phase(marl_ctx* c) {
     if (c->n == 0 && !c->n_on_device) return MARL_OK;
     c->c4_valid = false;  // the scatter writes every species
     CellLaunch a = cell_launch(c);
-    // When every cell gets a lane at once and nothing else needs the table's
-    // schedule this phase (no surrogate, no dependency hold, population on
-    // the host), the cell kernel computes each cell's schedule while staging
-    // it, and the schedule kernel is skipped.  The table's schedule is then
+    // When nothing else needs the table's schedule this phase (no surrogate, no
+    // dependency hold), the four-lane loop computes each cell's schedule while
+    // staging it, as the lane-per-cell loop does when every cell gets a lane at
+    // once, and the schedule kernel is skipped.  The table's schedule is then
     // left stale (schedule_dirty stays set) for any later phase that reads it.
-    const bool schedule_here = (!c->surr || c->surr_mode == MARL_SURR_OFF) && c->hold_cell < 0 &&
-                               !c->n_on_device && cell_tick_covers(c->n, c->cell_lanes, c->num_sms);
+    const bool plain = !c->surr || c->surr_mode == MARL_SURR_OFF;
+    const CellRoute route = plain ? cell_tick_route(a, c->num_sms) : CellRoute::kLane;
+    if (route == CellRoute::kEither && c->hold_cell < 0) a.split = cell_quad_limit(c->num_sms);
+    const bool schedule_here =
+        plain && c->hold_cell < 0 &&
+        (route != CellRoute::kLane || (!c->n_on_device && cell_tick_covers(c->n, c->cell_lanes, c->num_sms)));
     a.k.schedule_here = schedule_here ? 1u : 0u;
-    if (c->schedule_dirty && !schedule_here) {
+    if (c->schedule_dirty && (!schedule_here || a.split)) {
         CK(launch_cell_schedule(a, c->stream));
-        c->schedule_dirty = false;
+        c->schedule_dirty = a.split != 0;  // with a split the kernel may have returned at once
         ++c->launches;
     }
     if (c->hold_cell >= 0) {  // marl_ctx_test_hold_dependency: this phase only
@@ -345,7 +349,7 @@ marl_status enqueue_cell_phase(marl_ctx* c) {
         a.sv.ld = c->t.cap;
     }
     CK(launch_cell_tick(a, c->num_sms, c->stream));
-    ++c->launches;
+    c->launches += a.split ? 2 : 1;
     if (a.mode == kModeGated || a.mode == kModeTrusted) {
         CK(launch_surrogate_count(c->surr_status, c->surr_err, c->n, c->surr_counters,
                                   reinterpret_cast<uint32_t*>(c->surr_counters + 4), c->stream));

@@ -114,10 +114,12 @@ cudaError_t launch_diffuse_batch(int tile, const RunDesc* runs, const CUtensorMa
                                  uint32_t* err, cudaStream_t s);
 cudaError_t launch_light_batch(const RunDesc* runs, const int4* items, int n_items, const FieldConsts& k, int parity,
                                int use_c4, cudaStream_t s);
-cudaError_t launch_cell_schedule_batch(const RunDesc* runs, int n_runs, int num_sms, cudaStream_t s);
-// mode: kModePlain, kModeGated or kModeTrusted (the runs' sv hold the arrays).
+// split (here and in launch_cell_tick_batch): as CellLaunch::split.
+cudaError_t launch_cell_schedule_batch(const RunDesc* runs, int n_runs, uint32_t split, int num_sms, cudaStream_t s);
+// mode: kModePlain, kModeGated or kModeTrusted (the runs' sv hold the arrays);
+// total_cap: the sum of the runs' capacities.
 cudaError_t launch_cell_tick_batch(const RunDesc* runs, int n_runs, BatchScalars* bs, const CellConsts& k, int parity,
-                                   int num_sms, int mode, cudaStream_t s);
+                                   int num_sms, int mode, uint64_t total_cap, cudaStream_t s);
 // Surrogate pre-pass over the first `total` cells of the batch (global rows):
 // xt [16][ld] and standardised BF16 features X [rows][128].
 cudaError_t launch_surrogate_prepass_batch(const RunDesc* runs, int n_runs, uint32_t total, const CellConsts& k,
@@ -153,6 +155,10 @@ struct CellLaunch {
     uint32_t* ticket;
     uint32_t* err;
     float* act = nullptr;  // receptor activations [8][cap] of the cells updated (nullable)
+    // Device-resident count: populations up to `split` are the four-lane loop's,
+    // larger ones the schedule kernel's and the lane-per-cell loop's; each of
+    // the kernels looks and returns when it is not its turn.  0: no split.
+    uint32_t split = 0;
 };
 
 cudaError_t launch_cell_schedule(const CellLaunch& a, cudaStream_t s);
@@ -162,6 +168,12 @@ cudaError_t launch_cell_schedule(const CellLaunch& a, cudaStream_t s);
 cudaError_t launch_hold_dependency(const CellTable& t, uint32_t cell, int face, uint32_t slot, uint32_t* err,
                                    cudaStream_t s);
 cudaError_t launch_cell_tick(const CellLaunch& a, int num_sms, cudaStream_t s);
+// Which cell loop a launch takes: four lanes per cell, one lane per cell, or
+// (a device-resident count that may be either) both, one of which returns.
+enum class CellRoute { kLane, kQuad, kEither };
+CellRoute cell_tick_route(const CellLaunch& a, int num_sms);
+// The largest population of the four-lane loop.
+uint32_t cell_quad_limit(int num_sms);
 // Whether the plain cell kernel's grid gives each of n cells its own lane at
 // once (warp tickets); then the kernel can compute the schedule itself.
 bool cell_tick_covers(uint32_t n, uint32_t lanes, int num_sms);
