@@ -932,7 +932,11 @@ marl_status marl_batch_create(const marl_run_spec* specs, uint32_t n_runs, const
         if (e != cudaSuccess) return bail(cuda_fail(e, "cell upload"));
         b->h2d += cells[r].size() * sizeof(marl_cell);
     }
-    if ((st = plan_tiles(b, 0, 16, b->stream))) return bail(st);
+    std::vector<Grid> grids;
+    for (const auto& R : b->runs) grids.push_back(R.g);
+    int tile, zc;
+    default_diffusion_tile(grids.data(), (int)grids.size(), sms, &tile, &zc);
+    if ((st = plan_tiles(b, tile, zc, b->stream))) return bail(st);
     // Everything issued on the legacy default stream above (copies, memsets)
     // completes before any launch on the batch's non-blocking stream.
     if ((e = cudaDeviceSynchronize()) != cudaSuccess) return bail(cuda_fail(e, "marl_batch_create sync"));

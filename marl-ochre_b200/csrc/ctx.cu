@@ -529,7 +529,9 @@ marl_status marl_ctx_create(int32_t gx, int32_t gy, int32_t gz, const marl_sim_p
     c->n = 0;
     c->epoch = 0;
     c->schedule_dirty = true;
-    if (!plan_diffusion(&c->plan, c->field[0], c->field[1], c->mask, c->g, 0, 16)) {
+    int tile, zc;
+    default_diffusion_tile(&c->g, 1, sms, &tile, &zc);
+    if (!plan_diffusion(&c->plan, c->field[0], c->field[1], c->mask, c->g, tile, zc)) {
         ctx_free(c);
         return fail(MARL_ERR_CUDA, "cuTensorMapEncodeTiled failed for the field/mask tensor maps");
     }
@@ -1032,7 +1034,9 @@ marl_status marl_diffuse_device(float* field_dev, float* scratch_dev, const uint
     };
     if (e != cudaSuccess) return bail(cuda_fail(e, "occupancy mask"));
     DiffusionPlan plan;
-    if (!plan_diffusion(&plan, field_dev, scratch_dev, mask, g, 0, 16))
+    int tile, zc;
+    default_diffusion_tile(&g, 1, sms, &tile, &zc);
+    if (!plan_diffusion(&plan, field_dev, scratch_dev, mask, g, tile, zc))
         return bail(fail(MARL_ERR_CUDA, "cuTensorMapEncodeTiled failed"));
     int cur = 0;  // 0: field_dev holds the live state, 1: scratch_dev does
     for (uint32_t i = 0; i < substeps && e == cudaSuccess; ++i) {

@@ -816,6 +816,51 @@ bool encode_mask_map(CUtensorMap* m, const uint8_t* base, const Grid& g, int tx,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The tile and z-chunk of a launch over the given grids when nobody chose one.
+// The time of a launch goes as the number of waves of resident blocks times the
+// planes a block walks (its own and about 0.7 of a plane of start-up), at
+// nearly the same rate for the two 4-row tiles: tile 2 (four stages, TMA
+// stores, 7 blocks an SM) and tile 8 (three stages, direct stores, 10 blocks,
+// a plane taking 1.23 times as long).  The rule takes the smallest product; it
+// was within 3.4 % on average (at worst 19 %, a grid of 2,048 voxels) of the
+// best of 12 tiles x 14 z-chunks timed on 22 grids of 2k to 8.4M voxels.  A
+// single grid of more than four waves of tile 8 is bound by DRAM, where the
+// 8-row tile's smaller halo counts: tile 0 with 24 planes was the best of all
+// there.  Tile 0 with 16 planes, the fixed choice before: 12.6 us a substep at
+// 64x64x32 against 5.5, 16.4 against 8.0 at 64x64x64, 22.8 against 20.7 at
+// 128x128x64, 57.1 against 51.7 at 192x160x96, 92.7 against 88.5 at
+// 209x184x131, 146.9 against 144.0 at 256x256x128.
+void default_diffusion_tile(const Grid* grids, int n, int num_sms, int* tile, int* zc) {
+    struct {
+        int tile, blocks_per_sm;
+        double plane;
+    } const forms[] = {{2, 7, 0.81}, {8, 10, 1.0}};
+    int deepest = 1;
+    for (int i = 0; i < n; ++i) deepest = grids[i].Z > deepest ? grids[i].Z : deepest;
+    double best = 1e300;
+    *tile = 8;
+    *zc = 16;
+    for (const auto& f : forms) {
+        int tx, ty;
+        diffusion_tile_shape(f.tile, &tx, &ty);
+        for (int c = 2; c <= 32 && (c == 2 || c <= deepest); ++c) {
+            uint64_t blocks = 0;
+            for (int i = 0; i < n; ++i) {
+                const Grid& g = grids[i];
+                blocks += (uint64_t)((g.X + tx - 1) / tx) * ((g.Y + ty - 1) / ty) * ((g.Z + c - 1) / c);
+            }
+            const uint64_t slots = (uint64_t)f.blocks_per_sm * num_sms;
+            const double cost = (double)((blocks + slots - 1) / slots) * (c + 0.73) * f.plane;
+            if (cost < best) best = cost, *tile = f.tile, *zc = c;
+            if (n == 1 && f.tile == 8 && c == 12 && blocks > 4 * slots) {
+                *tile = 0;
+                *zc = 24;
+                return;
+            }
+        }
+    }
+}
+
 bool plan_diffusion(DiffusionPlan* plan, const float* a, const float* b, const uint8_t* mask, const Grid& g,
                     int tile, int zc) {
     int tx, ty;

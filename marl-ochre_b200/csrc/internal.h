@@ -26,6 +26,8 @@ int diffusion_tile_count();
 void diffusion_tile_shape(int tile, int* tx, int* ty);
 bool encode_field_map(CUtensorMap* m, const float* base, const Grid& g, int box_voxels, int box_rows);
 bool encode_mask_map(CUtensorMap* m, const uint8_t* base, const Grid& g, int tx, int ty);
+// Tile and z-chunk for a launch over n grids (a rule; the autotuner measures).
+void default_diffusion_tile(const Grid* grids, int n, int num_sms, int* tile, int* zc);
 bool plan_diffusion(DiffusionPlan* plan, const float* a, const float* b, const uint8_t* mask, const Grid& g,
                     int tile, int zc);
 

@@ -98,7 +98,9 @@ extern "C" marl_status marl_diffuse_device_noalloc(float* field_dev, const uint8
     if (!in_place && (e = launch_repack_mask(occupancy_dev, mask, g, s)) != cudaSuccess)
         return cuda_fail(e, "repack occupancy");
     DiffusionPlan plan;
-    if (!plan_diffusion(&plan, field_dev, scratch, in_place ? occupancy_dev : mask, g, 0, 16))
+    int tile, zc;
+    default_diffusion_tile(&g, 1, sms, &tile, &zc);
+    if (!plan_diffusion(&plan, field_dev, scratch, in_place ? occupancy_dev : mask, g, tile, zc))
         return fail(MARL_ERR_CUDA, "cuTensorMapEncodeTiled failed");
     int cur = 0;  // 0: field_dev holds the live state, 1: the scratch copy does
     for (uint32_t i = 0; i < substeps; ++i) {
