@@ -27,7 +27,8 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 # Per-file extra flags (default: exact IEEE float semantics).
 EXACT = ["-fmad=false", "-prec-div=true", "-prec-sqrt=true", "-ftz=false"]
-FLAGS = {"mlp.cu": ["-prec-div=true", "-prec-sqrt=true", "-ftz=false"]}  # MLP: FMA contraction allowed
+MLP = ["-prec-div=true", "-prec-sqrt=true", "-ftz=false"]  # FMA contraction allowed
+FLAGS = {"mlp.cu": MLP, "mlp_train.cu": MLP}
 
 
 def nvcc() -> str:

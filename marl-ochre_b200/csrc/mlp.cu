@@ -1,5 +1,6 @@
-// Tensor-core kernels of the reaction surrogate: a tcgen05 GEMM with the MLP's
-// epilogues, the loss, batch gathering, Adam, and the feature statistics.
+// Inference kernels of the reaction surrogate (a tcgen05 GEMM per layer, and the
+// whole network in one persistent kernel), the feature statistics and the
+// initial weights.  Training is in mlp_train.cu.
 //
 // GEMM form: C[M][N] = A[M][K] * B[N][K]^T with A and B BF16, both K-major
 // (row-major with K contiguous), FP32 accumulation in tensor memory.  One CTA
@@ -11,110 +12,20 @@
 // tcgen05.commit onto the stage's mbarrier.  The epilogue reads the
 // accumulator with tcgen05.ld (warp w owns TMEM lanes 32w..32w+31, i.e. rows
 // of the tile) and applies one of:
-//   BIAS_GELU  h = gelu(acc + b): BF16 out, optional BF16 transpose, FP32 z
-//              (BIAS_GELU_FAST: the same with the hardware tanh, for inference)
-//   BIAS_OUT   y = (acc + b) * scale + shift: FP32 out, row- or column-major
-//   GELU_BWD   dz = acc * gelu'(z): BF16 out and transpose, column sums
-//   ATOMIC     out[m][n] += acc (split-K weight gradients), or out[n][m]
-// All three training GEMM shapes (forward, input gradient, weight gradient)
-// are this one form, given transposed copies that the epilogues write.
+//   BIAS_GELU_FAST  h = gelu(acc + b) with the hardware tanh: BF16 out
+//   BIAS_OUT        y = (acc + b) * scale + shift: FP32 out, row- or column-major
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include "common.cuh"
 #include "kernel_setup.h"
 #include "mlp.h"
+#include "mlp_umma.cuh"
 
 namespace marl {
 namespace mlp {
 
-constexpr int kBM = 128;
-constexpr int kBK = 64;
 constexpr int kGemmThreads = 128;
-
-__device__ __forceinline__ void cp_async16_zfill(uint32_t dst, const void* src, uint32_t src_bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(src_bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit_wait_all() {
-    asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
-}
-
-// Shared-memory matrix descriptor: K-major, 128-byte swizzle, 8-row groups
-// 1024 bytes apart (SBO), leading offset unused for this layout (1), version 1.
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
-    uint64_t d = (uint64_t)((saddr & 0x3FFFFu) >> 4);
-    d |= (uint64_t)1u << 16;
-    d |= (uint64_t)(1024u >> 4) << 32;
-    d |= (uint64_t)1u << 46;
-    d |= (uint64_t)2u << 61;
-    return d;
-}
-
-// Instruction descriptor, kind::f16: FP32 accumulator, BF16 A and B, both
-// K-major, N >> 3 at bit 17, M >> 4 at bit 24.
-__host__ __device__ constexpr uint32_t idesc_bf16(int M, int N) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
-}
-
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
-                                          uint32_t accumulate) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-        : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-                 : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
-    uint32_t r[16];
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-        : "r"(taddr));
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(r[i]);
-}
-
-__device__ __forceinline__ float gelu_t(float z, float& t) {
-    const float u = 0.7978845608028654f * (z + 0.044715f * z * z * z);
-    t = tanhf(u);
-    return 0.5f * z * (1.0f + t);
-}
-// Inference form: the hardware tanh approximation (MUFU), max relative error
-// about 2^-11, below the BF16 rounding the activation goes through next.
-__device__ __forceinline__ float gelu_fast(float z) {
-    const float u = 0.7978845608028654f * (z + 0.044715f * z * z * z);
-    float t;
-    asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(u));
-    return 0.5f * z * (1.0f + t);
-}
-__device__ __forceinline__ float gelu_grad(float z) {
-    const float u = 0.7978845608028654f * (z + 0.044715f * z * z * z);
-    const float t = tanhf(u);
-    return 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * 0.7978845608028654f * (1.0f + 3.0f * 0.044715f * z * z);
-}
-
-__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
-    const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<const uint32_t*>(&h);
-}
-
-// Bounded mbarrier wait for the tensor-core commit of a stage.
-__device__ __forceinline__ bool wait_commit(uint64_t* bar, uint32_t parity, uint32_t* err) {
-    if (mbar_wait_bounded(bar, parity)) return true;
-    if (err) atomicOr(err, kErrTimeoutMbar);
-    return false;
-}
 
 template <int BN, int EPI>
 __global__ void __launch_bounds__(kGemmThreads) k_gemm(const __grid_constant__ GemmArgs a) {
@@ -131,9 +42,7 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(const __grid_constant__ G
     const uint32_t base = (smem_u32(gsm_raw) + 1023u) & ~1023u;  // swizzle atoms need 1024-byte alignment
     const int m0 = blockIdx.x * kBM;
     const int n0 = blockIdx.y * BN;
-    const int k_begin = blockIdx.z * a.k_per_split;
-    const int k_end = min(a.K, k_begin + a.k_per_split);
-    const int nch = (k_end - k_begin) / kBK;
+    const int nch = a.K / kBK;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
@@ -157,7 +66,7 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(const __grid_constant__ G
         const int s = c & 1;
         if (c >= 2) ok = wait_commit(&bars[s], ((c - 2) >> 1) & 1, a.err) && ok;
         const uint32_t sa = base + s * kStage, sb = sa + kStageA;
-        const int k0 = k_begin + c * kBK;
+        const int k0 = c * kBK;
         // A: 128 rows x 8 pieces of 16 bytes; rows beyond M are zero-filled.
 #pragma unroll
         for (int i = 0; i < (kBM * 8) / kGemmThreads; ++i) {
@@ -198,34 +107,16 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(const __grid_constant__ G
         float v[16];
         tmem_ld16(t_lane + cb, v);
         const int n = n0 + cb;
-        if constexpr (EPI == EPI_BIAS_GELU || EPI == EPI_BIAS_GELU_FAST) {
+        if constexpr (EPI == EPI_BIAS_GELU_FAST) {
             float h[16];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                const float z = v[i] + a.bias[n + i];
-                if constexpr (EPI == EPI_BIAS_GELU_FAST) {
-                    h[i] = gelu_fast(z);
-                } else {
-                    float t;
-                    h[i] = gelu_t(z, t);
-                }
-                v[i] = z;
-            }
+            for (int i = 0; i < 16; ++i) h[i] = gelu_fast(v[i] + a.bias[n + i]);
             if (row_ok) {
                 uint4* o = reinterpret_cast<uint4*>(a.out_bf + (size_t)row * a.ldo + n);
                 o[0] = make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]),
                                   pack_bf16(h[6], h[7]));
                 o[1] = make_uint4(pack_bf16(h[8], h[9]), pack_bf16(h[10], h[11]), pack_bf16(h[12], h[13]),
                                   pack_bf16(h[14], h[15]));
-                if (a.out_f) {
-                    float4* zf = reinterpret_cast<float4*>(a.out_f + (size_t)row * a.ldf + n);
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) zf[i] = make_float4(v[4 * i], v[4 * i + 1], v[4 * i + 2], v[4 * i + 3]);
-                }
-                if (a.out_t) {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) a.out_t[(size_t)(n + i) * a.ldt + row] = __float2bfloat16_rn(h[i]);
-                }
             }
         } else if constexpr (EPI == EPI_BIAS_OUT) {
             if (row_ok) {
@@ -239,47 +130,6 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(const __grid_constant__ G
                         a.out_f[(size_t)row * a.ldf + n + i] = y;
                 }
             }
-        } else if constexpr (EPI == EPI_GELU_BWD) {
-            float d[16];
-            if (row_ok) {
-                const float4* zp = reinterpret_cast<const float4*>(a.z_in + (size_t)row * a.ldz + n);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float4 z = zp[i];
-                    d[4 * i] = v[4 * i] * gelu_grad(z.x);
-                    d[4 * i + 1] = v[4 * i + 1] * gelu_grad(z.y);
-                    d[4 * i + 2] = v[4 * i + 2] * gelu_grad(z.z);
-                    d[4 * i + 3] = v[4 * i + 3] * gelu_grad(z.w);
-                }
-                uint4* o = reinterpret_cast<uint4*>(a.out_bf + (size_t)row * a.ldo + n);
-                o[0] = make_uint4(pack_bf16(d[0], d[1]), pack_bf16(d[2], d[3]), pack_bf16(d[4], d[5]),
-                                  pack_bf16(d[6], d[7]));
-                o[1] = make_uint4(pack_bf16(d[8], d[9]), pack_bf16(d[10], d[11]), pack_bf16(d[12], d[13]),
-                                  pack_bf16(d[14], d[15]));
-#pragma unroll
-                for (int i = 0; i < 16; ++i) a.out_t[(size_t)(n + i) * a.ldt + row] = __float2bfloat16_rn(d[i]);
-            } else {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) d[i] = 0.0f;
-            }
-            // bias gradient: column sums of dz over the tile's rows
-#pragma unroll
-            for (int i = 0; i < 16; ++i) {
-                float sum = d[i];
-#pragma unroll
-                for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xFFFFFFFFu, sum, o);
-                if (lane == 0 && a.colsum) atomicAdd(&a.colsum[n + i], sum);
-            }
-        } else {  // EPI_ATOMIC
-            if (row_ok) {
-#pragma unroll
-                for (int i = 0; i < 16; ++i) {
-                    if (a.out_col_major)
-                        atomicAdd(&a.out_f[(size_t)(n + i) * a.ldf + row], v[i]);
-                    else
-                        atomicAdd(&a.out_f[(size_t)row * a.ldf + n + i], v[i]);
-                }
-            }
         }
     }
     tc_fence_before();
@@ -289,34 +139,20 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(const __grid_constant__ G
 }
 
 template <int BN, int EPI>
-static cudaError_t launch_one(const GemmArgs& a, int splits, cudaStream_t s) {
+static cudaError_t launch_one(const GemmArgs& a, cudaStream_t s) {
     constexpr int smem = 2 * (kBM * 128 + BN * 128) + 1024;
     static std::atomic<int> setup[kSetupDevices];
     cudaError_t e = set_smem_once(setup, k_gemm<BN, EPI>, smem);
     if (e != cudaSuccess) return e;
-    dim3 grid((a.M + kBM - 1) / kBM, a.N / BN, splits);
+    dim3 grid((a.M + kBM - 1) / kBM, a.N / BN);
     k_gemm<BN, EPI><<<grid, kGemmThreads, smem, s>>>(a);
     return cudaGetLastError();
 }
 
 cudaError_t launch_gemm(const GemmArgs& a, int bn, int epi, cudaStream_t s) {
     if (a.M <= 0 || a.K <= 0 || a.K % kBK || a.N % bn || a.lda % 8 || a.ldb % 8) return cudaErrorInvalidValue;
-    const int kps = a.k_per_split > 0 ? a.k_per_split : a.K;
-    if (kps % kBK) return cudaErrorInvalidValue;
-    const int splits = (a.K + kps - 1) / kps;
-    if (splits > 1 && epi != EPI_ATOMIC) return cudaErrorInvalidValue;
-    GemmArgs b = a;
-    b.k_per_split = kps;
-#define MARL_GEMM_CASE(BNV, EPIV) \
-    if (bn == BNV && epi == EPIV) return launch_one<BNV, EPIV>(b, splits, s);
-    MARL_GEMM_CASE(256, EPI_BIAS_GELU)
-    MARL_GEMM_CASE(256, EPI_BIAS_GELU_FAST)
-    MARL_GEMM_CASE(16, EPI_BIAS_OUT)
-    MARL_GEMM_CASE(256, EPI_GELU_BWD)
-    MARL_GEMM_CASE(256, EPI_ATOMIC)
-    MARL_GEMM_CASE(128, EPI_ATOMIC)
-    MARL_GEMM_CASE(16, EPI_ATOMIC)
-#undef MARL_GEMM_CASE
+    if (bn == 256 && epi == EPI_BIAS_GELU_FAST) return launch_one<256, EPI_BIAS_GELU_FAST>(a, s);
+    if (bn == 16 && epi == EPI_BIAS_OUT) return launch_one<16, EPI_BIAS_OUT>(a, s);
     return cudaErrorInvalidValue;
 }
 
@@ -536,141 +372,6 @@ cudaError_t launch_mlp_fused(const FusedArgs& a, int num_sms, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     const int ntiles = (a.M + kBM - 1) / kBM;
     k_mlp_fused<<<ntiles < num_sms ? ntiles : num_sms, kFusedThreads, kFusedSmem, s>>>(a);
-    return cudaGetLastError();
-}
-
-// ------------------------------------------------------------- loss -----
-// dY = 2 (y - t) / (B * 16) as BF16 [B][64] (columns 16..63 zero) and its
-// transpose [16][B]; bias gradient of the output layer and the loss sum.
-__global__ void k_loss(const float* __restrict__ y, const float* __restrict__ t, uint32_t B,
-                       __nv_bfloat16* __restrict__ dy, __nv_bfloat16* __restrict__ dyt, float* __restrict__ db3,
-                       float* __restrict__ loss_sum) {
-    __shared__ float s_db[16];
-    __shared__ float s_loss;
-    if (threadIdx.x < 16) s_db[threadIdx.x] = 0.0f;
-    if (threadIdx.x == 0) s_loss = 0.0f;
-    __syncthreads();
-    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    float l = 0.0f;
-    const float sc = 2.0f / ((float)B * 16.0f);
-    if (r < B) {
-        uint32_t w[8];
-        for (int i = 0; i < 16; i += 2) {
-            const float e0 = y[(size_t)r * 16 + i] - t[(size_t)r * 16 + i];
-            const float e1 = y[(size_t)r * 16 + i + 1] - t[(size_t)r * 16 + i + 1];
-            l += e0 * e0 + e1 * e1;
-            const float g0 = e0 * sc, g1 = e1 * sc;
-            w[i >> 1] = pack_bf16(g0, g1);
-            dyt[(size_t)i * B + r] = __float2bfloat16_rn(g0);
-            dyt[(size_t)(i + 1) * B + r] = __float2bfloat16_rn(g1);
-            atomicAdd(&s_db[i], g0);
-            atomicAdd(&s_db[i + 1], g1);
-        }
-        uint4* o = reinterpret_cast<uint4*>(dy + (size_t)r * 64);
-        o[0] = make_uint4(w[0], w[1], w[2], w[3]);
-        o[1] = make_uint4(w[4], w[5], w[6], w[7]);
-        for (int i = 2; i < 8; ++i) o[i] = make_uint4(0, 0, 0, 0);
-        atomicAdd(&s_loss, l);
-    }
-    __syncthreads();
-    if (threadIdx.x < 16) atomicAdd(&db3[threadIdx.x], s_db[threadIdx.x]);
-    if (threadIdx.x == 0) atomicAdd(loss_sum, s_loss);
-}
-
-cudaError_t launch_loss(const float* y, const float* t, uint32_t B, __nv_bfloat16* dy, __nv_bfloat16* dyt,
-                        float* db3, float* loss_sum, cudaStream_t s) {
-    k_loss<<<(B + 255) / 256, 256, 0, s>>>(y, t, B, dy, dyt, db3, loss_sum);
-    return cudaGetLastError();
-}
-
-// ------------------------------------------------------------ batches ----
-__device__ __forceinline__ uint64_t mix64(uint64_t z) {  // splitmix64 finaliser
-    z += 0x9E3779B97F4A7C15ull;
-    z = (z ^ (z >> 30)) * 0xBF58476D1CE4E5B9ull;
-    z = (z ^ (z >> 27)) * 0x94D049BB133111EBull;
-    return z ^ (z >> 31);
-}
-
-// Row r of the batch is training row hash(seed, step, r) mod n_rows: copies
-// its standardised input (BF16 [128]) and target (FP32 [16]), and writes the
-// input transposed ([128][B]) for the first layer's weight gradient.
-__global__ void k_gather_batch(const __nv_bfloat16* __restrict__ X, const float* __restrict__ T, uint32_t n_rows,
-                               uint64_t seed, uint64_t step, uint32_t B, __nv_bfloat16* __restrict__ xb,
-                               __nv_bfloat16* __restrict__ xbt, float* __restrict__ tb) {
-    const uint32_t r = blockIdx.x;
-    if (r >= B) return;
-    const uint32_t src = (uint32_t)(mix64(seed ^ mix64(step * 0x100000001B3ull + r)) % n_rows);
-    const int i = threadIdx.x;  // 0..127
-    const __nv_bfloat16 v = X[(size_t)src * kInPad + i];
-    xb[(size_t)r * kInPad + i] = v;
-    xbt[(size_t)i * B + r] = v;
-    if (i < 16) tb[(size_t)r * 16 + i] = T[(size_t)src * 16 + i];
-}
-
-cudaError_t launch_gather_batch(const __nv_bfloat16* X, const float* T, uint32_t n_rows, uint64_t seed, uint64_t step,
-                                uint32_t B, __nv_bfloat16* xb, __nv_bfloat16* xbt, float* tb, cudaStream_t s) {
-    k_gather_batch<<<B, kInPad, 0, s>>>(X, T, n_rows, seed, step, B, xb, xbt, tb);
-    return cudaGetLastError();
-}
-
-// Transposes a host-provided batch (gradient checks): xbt[i][r] = xb[r][i].
-__global__ void k_transpose_batch(const __nv_bfloat16* __restrict__ xb, uint32_t B, __nv_bfloat16* __restrict__ xbt) {
-    const uint32_t r = blockIdx.x;
-    xbt[(size_t)threadIdx.x * B + r] = xb[(size_t)r * kInPad + threadIdx.x];
-}
-
-cudaError_t launch_transpose_batch(const __nv_bfloat16* xb, uint32_t B, __nv_bfloat16* xbt, cudaStream_t s) {
-    k_transpose_batch<<<B, kInPad, 0, s>>>(xb, B, xbt);
-    return cudaGetLastError();
-}
-
-// --------------------------------------------------------------- Adam ----
-// FP32 master parameters p (flat, MARL_SURR_PARAMS) updated from gradients g;
-// then the BF16 copies the GEMMs read: W1, W2, W3, W2^T and W3^T (padded to
-// 64 columns).
-__global__ void k_adam(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
-                       float* __restrict__ v, uint32_t n, float lr, float b1, float b2, float eps, float bc1,
-                       float bc2) {
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * gi;
-        const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        p[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-    }
-}
-
-__global__ void k_weights_bf16(const float* __restrict__ p, __nv_bfloat16* __restrict__ w1,
-                               __nv_bfloat16* __restrict__ w2, __nv_bfloat16* __restrict__ w3,
-                               __nv_bfloat16* __restrict__ w2t, __nv_bfloat16* __restrict__ w3t) {
-    const float* W1 = p + kOffW1;
-    const float* W2 = p + kOffW2;
-    const float* W3 = p + kOffW3;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < kHid * kHid; i += gridDim.x * blockDim.x) {
-        const uint32_t o = i / kHid, k = i % kHid;
-        w2[i] = __float2bfloat16_rn(W2[i]);
-        w2t[(size_t)k * kHid + o] = __float2bfloat16_rn(W2[i]);
-        if (i < kHid * kInPad) w1[i] = __float2bfloat16_rn(W1[i]);
-        if (i < kOut * kHid) w3[i] = __float2bfloat16_rn(W3[i]);
-        if (i < kHid * kOutPad) {
-            const uint32_t hi = i / kOutPad, oo = i % kOutPad;  // w3t[hi][oo] = W3[oo][hi]
-            w3t[i] = __float2bfloat16_rn(oo < kOut ? W3[(size_t)oo * kHid + hi] : 0.0f);
-        }
-    }
-}
-
-cudaError_t launch_adam(float* p, const float* g, float* m, float* v, float lr, float b1, float b2, float eps,
-                        uint64_t t, cudaStream_t s) {
-    const float bc1 = 1.0f - (float)pow((double)b1, (double)t);
-    const float bc2 = 1.0f - (float)pow((double)b2, (double)t);
-    k_adam<<<256, 256, 0, s>>>(p, g, m, v, kParams, lr, b1, b2, eps, bc1, bc2);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_weights_bf16(const float* p, __nv_bfloat16* w1, __nv_bfloat16* w2, __nv_bfloat16* w3,
-                                __nv_bfloat16* w2t, __nv_bfloat16* w3t, cudaStream_t s) {
-    k_weights_bf16<<<256, 256, 0, s>>>(p, w1, w2, w3, w2t, w3t);
     return cudaGetLastError();
 }
 

@@ -14,7 +14,6 @@ constexpr int kIn = MARL_SURR_FEATURES;  // 93 features
 constexpr int kInPad = 128;              // first-layer K, zero-padded
 constexpr int kHid = 256;
 constexpr int kOut = 16;
-constexpr int kOutPad = 64;              // K of the output layer's input-gradient GEMM
 
 // Flat parameter layout (FP32 master copy, gradients, Adam moments).
 constexpr uint32_t kOffW1 = 0;
@@ -35,7 +34,7 @@ __device__ __forceinline__ float feature_transform(int f, float v) {
 }
 #endif
 
-enum Epi : int { EPI_BIAS_GELU = 0, EPI_BIAS_OUT = 1, EPI_GELU_BWD = 2, EPI_ATOMIC = 3, EPI_BIAS_GELU_FAST = 4 };
+enum Epi : int { EPI_BIAS_OUT, EPI_BIAS_GELU_FAST };
 
 struct GemmArgs {
     const __nv_bfloat16* A = nullptr;  // [M][lda], K contiguous
@@ -43,20 +42,14 @@ struct GemmArgs {
     const __nv_bfloat16* B = nullptr;  // [N][ldb], K contiguous
     int ldb = 0;
     int M = 0, N = 0, K = 0;
-    int k_per_split = 0;               // 0: whole K in one CTA (split-K only with EPI_ATOMIC)
     const float* bias = nullptr;       // [N]
     const float* scale = nullptr;      // [N] optional (EPI_BIAS_OUT)
     const float* shift = nullptr;      // [N] with scale
     __nv_bfloat16* out_bf = nullptr;   // [M][ldo]
     int ldo = 0;
-    __nv_bfloat16* out_t = nullptr;    // [N][ldt] transposed BF16 copy
-    int ldt = 0;
-    float* out_f = nullptr;            // FP32 output / pre-activation / atomic target
+    float* out_f = nullptr;            // FP32 output (EPI_BIAS_OUT)
     int ldf = 0;
-    int out_col_major = 0;             // out_f as [N][ldf] (EPI_BIAS_OUT, EPI_ATOMIC)
-    const float* z_in = nullptr;       // [M][ldz] pre-activation (EPI_GELU_BWD)
-    int ldz = 0;
-    float* colsum = nullptr;           // [N] column sums of the output (EPI_GELU_BWD)
+    int out_col_major = 0;             // out_f as [N][ldf]
     uint32_t* err = nullptr;           // kErr* bits on a wait timeout
 };
 
@@ -75,17 +68,43 @@ struct FusedArgs {
 };
 cudaError_t launch_mlp_fused(const FusedArgs& a, int num_sms, cudaStream_t s);
 
-// bn: 16, 128 or 256 (the instantiated tile widths for each epilogue).
+// (bn, epi): (256, EPI_BIAS_GELU_FAST) or (16, EPI_BIAS_OUT).
 cudaError_t launch_gemm(const GemmArgs& a, int bn, int epi, cudaStream_t s);
-cudaError_t launch_loss(const float* y, const float* t, uint32_t B, __nv_bfloat16* dy, __nv_bfloat16* dyt,
-                        float* db3, float* loss_sum, cudaStream_t s);
-cudaError_t launch_gather_batch(const __nv_bfloat16* X, const float* T, uint32_t n_rows, uint64_t seed, uint64_t step,
-                                uint32_t B, __nv_bfloat16* xb, __nv_bfloat16* xbt, float* tb, cudaStream_t s);
-cudaError_t launch_transpose_batch(const __nv_bfloat16* xb, uint32_t B, __nv_bfloat16* xbt, cudaStream_t s);
-cudaError_t launch_adam(float* p, const float* g, float* m, float* v, float lr, float b1, float b2, float eps,
-                        uint64_t t, cudaStream_t s);
+
+// One training step's buffers (B rows, a multiple of 128; see mlp_train.cu).
+struct TrainArgs {
+    uint32_t B = 0;
+    const __nv_bfloat16* X = nullptr;  // standardised rows [.][128]
+    const float* T = nullptr;          // their targets [.][16]
+    uint32_t n_rows = 0;               // batch row r is a hashed draw from [0, n_rows); 0: row r itself
+    uint64_t seed = 0, step = 0;       // of the draws
+    uint32_t* idx = nullptr;           // [B] the drawn rows
+    const __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr;
+    const float* p = nullptr;          // FP32 parameters (the biases are read)
+    __nv_bfloat16 *h1 = nullptr, *h2 = nullptr, *dy = nullptr, *dz2 = nullptr, *dz1 = nullptr;
+    float *d1 = nullptr, *d2 = nullptr;  // GELU' of the pre-activations [B][256]
+    float* y = nullptr;                // [B][16]
+    uint32_t split_rows = 0;           // rows of a weight-gradient partial sum (train_split_rows)
+    float* weight_part = nullptr;      // [splits][kParams]: the weights' partial sums
+    float* row_part = nullptr;         // [B / 128][kTrRowSums]: db1, db2, db3 and loss partial sums
+    float* g = nullptr;                // gradients (launch_train_gradients)
+    float* loss_sum = nullptr;
+    uint32_t* err = nullptr;
+};
+constexpr int kTrRowSums = 2 * kHid + kOut + 1;
+// Rows per partial sum of the weight gradients: 512, more where that would be
+// more than 32 sums.
+inline uint32_t train_split_rows(uint32_t B) { return 512u * ((B + 512u * 32u - 1u) / (512u * 32u)); }
+inline uint32_t train_splits(uint32_t B, uint32_t split_rows) { return (B + split_rows - 1) / split_rows; }
+cudaError_t launch_forward_backward(const TrainArgs& a, cudaStream_t s);
+// The gradients from the partial sums into a.g, or Adam's step with them (on the
+// FP32 parameters and their BF16 copies); both set *a.loss_sum.
+cudaError_t launch_train_gradients(const TrainArgs& a, cudaStream_t s);
+cudaError_t launch_train_update(const TrainArgs& a, float* p, float* m, float* v, float lr, float b1, float b2,
+                                float eps, uint64_t t, __nv_bfloat16* w1, __nv_bfloat16* w2, __nv_bfloat16* w3,
+                                cudaStream_t s);
 cudaError_t launch_weights_bf16(const float* p, __nv_bfloat16* w1, __nv_bfloat16* w2, __nv_bfloat16* w3,
-                                __nv_bfloat16* w2t, __nv_bfloat16* w3t, cudaStream_t s);
+                                cudaStream_t s);
 cudaError_t launch_raw_stats(const float* raw, uint32_t n, double* acc, cudaStream_t s);
 cudaError_t launch_standardise(const float* raw, uint32_t n, const float* norm, __nv_bfloat16* X, float* T,
                                cudaStream_t s);

@@ -1,21 +1,9 @@
 // C ABI of the learned reaction surrogate: pair store, standardisation,
-// training (forward, backward, Adam on the tcgen05 GEMM of mlp.cu),
-// evaluation, inference, and the hooks of a context's cell loop.
-//
-// Training step on a batch of B rows (all GEMMs C = A * B^T, K-major):
-//   h1 = gelu(x W1^T + b1)        A = x [B][128],     B = W1 [256][128]
-//   h2 = gelu(h1 W2^T + b2)       A = h1 [B][256],    B = W2 [256][256]
-//   y  = h2 W3^T + b3             A = h2 [B][256],    B = W3 [16][256]
-//   dy = 2 (y - t) / (16 B)
-//   dW3^T = h2^T dy               A = h2^T [256][B],  B = dy^T [16][B]
-//   dz2 = (dy W3) * gelu'(z2)     A = dy [B][64],     B = W3^T [256][64]
-//   dW2 = dz2^T h1                A = dz2^T [256][B], B = h1^T [256][B]
-//   dz1 = (dz2 W2) * gelu'(z1)    A = dz2 [B][256],   B = W2^T [256][256]
-//   dW1 = dz1^T x                 A = dz1^T [256][B], B = x^T [128][B]
-// Weight gradients use split-K with FP32 atomic accumulation; bias gradients
-// are column sums taken in the epilogues.
+// training (the step's kernels are in mlp_train.cu), evaluation, inference, and
+// the hooks of a context's cell loop.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <vector>
@@ -33,8 +21,6 @@ namespace marl {
         if (_e != cudaSuccess) return cuda_fail(_e, #expr);   \
     } while (0)
 
-static constexpr int kSplitK = 512;
-
 static void free_all(std::initializer_list<void*> ptrs) {
     for (void* p : ptrs)
         if (p) cudaFree(p);
@@ -43,26 +29,29 @@ static void free_all(std::initializer_list<void*> ptrs) {
 static marl_status ensure_work(marl_surrogate* s, uint32_t B) {
     if (B <= s->work_b) return MARL_OK;
     cudaStreamSynchronize(s->stream);
-    free_all({s->xb, s->xbt, s->h1, s->h1t, s->h2, s->h2t, s->dy, s->dyt, s->dz2, s->dz2t, s->dz1, s->dz1t, s->tb,
-              s->z1, s->z2, s->y});
+    free_all({s->xb, s->h1, s->h2, s->dy, s->dz2, s->dz1, s->tb, s->d1, s->d2, s->y, s->idx, s->weight_part,
+              s->row_part});
+    s->weight_part = s->row_part = nullptr;
+    s->xb = s->h1 = s->h2 = s->dy = s->dz2 = s->dz1 = nullptr;
+    s->tb = s->d1 = s->d2 = s->y = nullptr;
+    s->idx = nullptr;
     s->work_b = 0;
     const size_t b = B;
     SCK(cudaMalloc((void**)&s->xb, b * mlp::kInPad * 2));
-    SCK(cudaMalloc((void**)&s->xbt, b * mlp::kInPad * 2));
     SCK(cudaMalloc((void**)&s->h1, b * mlp::kHid * 2));
-    SCK(cudaMalloc((void**)&s->h1t, b * mlp::kHid * 2));
     SCK(cudaMalloc((void**)&s->h2, b * mlp::kHid * 2));
-    SCK(cudaMalloc((void**)&s->h2t, b * mlp::kHid * 2));
-    SCK(cudaMalloc((void**)&s->dy, b * mlp::kOutPad * 2));
-    SCK(cudaMalloc((void**)&s->dyt, b * mlp::kOut * 2));
+    SCK(cudaMalloc((void**)&s->dy, b * mlp::kOut * 2));
     SCK(cudaMalloc((void**)&s->dz2, b * mlp::kHid * 2));
-    SCK(cudaMalloc((void**)&s->dz2t, b * mlp::kHid * 2));
     SCK(cudaMalloc((void**)&s->dz1, b * mlp::kHid * 2));
-    SCK(cudaMalloc((void**)&s->dz1t, b * mlp::kHid * 2));
     SCK(cudaMalloc((void**)&s->tb, b * mlp::kOut * 4));
-    SCK(cudaMalloc((void**)&s->z1, b * mlp::kHid * 4));
-    SCK(cudaMalloc((void**)&s->z2, b * mlp::kHid * 4));
+    SCK(cudaMalloc((void**)&s->d1, b * mlp::kHid * 4));
+    SCK(cudaMalloc((void**)&s->d2, b * mlp::kHid * 4));
     SCK(cudaMalloc((void**)&s->y, b * mlp::kOut * 4));
+    SCK(cudaMalloc((void**)&s->idx, b * 4));
+    // A smaller batch may have as many partial sums (a split has at least 512 rows).
+    const size_t splits = std::min<size_t>((b + 511) / 512, 32);
+    SCK(cudaMalloc((void**)&s->weight_part, splits * mlp::kParams * 4));
+    SCK(cudaMalloc((void**)&s->row_part, b / 128 * mlp::kTrRowSums * 4));
     s->work_b = B;
     return MARL_OK;
 }
@@ -102,78 +91,17 @@ static marl_status gemm(const mlp::GemmArgs& a, int bn, int epi, cudaStream_t st
         if (_s != MARL_OK) return _s;               \
     } while (0)
 
-// Forward of the first two layers for training (keeps z, h and h^T).
-static marl_status forward_train(marl_surrogate* s, uint32_t B) {
-    cudaStream_t st = s->stream;
-    mlp::GemmArgs a;
-    a.err = s->d_err;
-    a.A = s->xb, a.lda = mlp::kInPad, a.B = s->w1, a.ldb = mlp::kInPad;
-    a.M = (int)B, a.N = mlp::kHid, a.K = mlp::kInPad;
-    a.bias = s->p + mlp::kOffB1, a.out_bf = s->h1, a.ldo = mlp::kHid, a.out_t = s->h1t, a.ldt = (int)B;
-    a.out_f = s->z1, a.ldf = mlp::kHid;
-    SST(gemm(a, 256, mlp::EPI_BIAS_GELU, st));
-    a.A = s->h1, a.lda = mlp::kHid, a.B = s->w2, a.ldb = mlp::kHid, a.K = mlp::kHid;
-    a.bias = s->p + mlp::kOffB2, a.out_bf = s->h2, a.out_t = s->h2t, a.out_f = s->z2;
-    SST(gemm(a, 256, mlp::EPI_BIAS_GELU, st));
-    mlp::GemmArgs o;
-    o.err = s->d_err;
-    o.A = s->h2, o.lda = mlp::kHid, o.B = s->w3, o.ldb = mlp::kHid;
-    o.M = (int)B, o.N = mlp::kOut, o.K = mlp::kHid;
-    o.bias = s->p + mlp::kOffB3, o.out_f = s->y, o.ldf = mlp::kOut;
-    SST(gemm(o, 16, mlp::EPI_BIAS_OUT, st));
-    return MARL_OK;
-}
-
-// Gradients into s->g (zeroed here) from the batch in xb/xbt/tb; the loss
-// sum is added to *loss_sum.
-static marl_status backward(marl_surrogate* s, uint32_t B, float* loss_sum) {
-    cudaStream_t st = s->stream;
-    SCK(cudaMemsetAsync(s->g, 0, (size_t)mlp::kParams * 4, st));
-    SCK(mlp::launch_loss(s->y, s->tb, B, s->dy, s->dyt, s->g + mlp::kOffB3, loss_sum, st));
-    const int kps = (int)B < kSplitK ? (int)B : kSplitK;
-    {  // dW3^T [256][16] = h2^T dy, stored as dW3 [16][256]
-        mlp::GemmArgs a;
-        a.err = s->d_err;
-        a.A = s->h2t, a.lda = (int)B, a.B = s->dyt, a.ldb = (int)B;
-        a.M = mlp::kHid, a.N = mlp::kOut, a.K = (int)B, a.k_per_split = kps;
-        a.out_f = s->g + mlp::kOffW3, a.ldf = mlp::kHid, a.out_col_major = 1;
-        SST(gemm(a, 16, mlp::EPI_ATOMIC, st));
-    }
-    {  // dz2 = (dy W3) * gelu'(z2)
-        mlp::GemmArgs a;
-        a.err = s->d_err;
-        a.A = s->dy, a.lda = mlp::kOutPad, a.B = s->w3t, a.ldb = mlp::kOutPad;
-        a.M = (int)B, a.N = mlp::kHid, a.K = mlp::kOutPad;
-        a.z_in = s->z2, a.ldz = mlp::kHid, a.out_bf = s->dz2, a.ldo = mlp::kHid, a.out_t = s->dz2t, a.ldt = (int)B;
-        a.colsum = s->g + mlp::kOffB2;
-        SST(gemm(a, 256, mlp::EPI_GELU_BWD, st));
-    }
-    {  // dW2 [256][256] = dz2^T h1
-        mlp::GemmArgs a;
-        a.err = s->d_err;
-        a.A = s->dz2t, a.lda = (int)B, a.B = s->h1t, a.ldb = (int)B;
-        a.M = mlp::kHid, a.N = mlp::kHid, a.K = (int)B, a.k_per_split = kps;
-        a.out_f = s->g + mlp::kOffW2, a.ldf = mlp::kHid;
-        SST(gemm(a, 256, mlp::EPI_ATOMIC, st));
-    }
-    {  // dz1 = (dz2 W2) * gelu'(z1)
-        mlp::GemmArgs a;
-        a.err = s->d_err;
-        a.A = s->dz2, a.lda = mlp::kHid, a.B = s->w2t, a.ldb = mlp::kHid;
-        a.M = (int)B, a.N = mlp::kHid, a.K = mlp::kHid;
-        a.z_in = s->z1, a.ldz = mlp::kHid, a.out_bf = s->dz1, a.ldo = mlp::kHid, a.out_t = s->dz1t, a.ldt = (int)B;
-        a.colsum = s->g + mlp::kOffB1;
-        SST(gemm(a, 256, mlp::EPI_GELU_BWD, st));
-    }
-    {  // dW1 [256][128] = dz1^T x
-        mlp::GemmArgs a;
-        a.err = s->d_err;
-        a.A = s->dz1t, a.lda = (int)B, a.B = s->xbt, a.ldb = (int)B;
-        a.M = mlp::kHid, a.N = mlp::kInPad, a.K = (int)B, a.k_per_split = kps;
-        a.out_f = s->g + mlp::kOffW1, a.ldf = mlp::kInPad;
-        SST(gemm(a, 128, mlp::EPI_ATOMIC, st));
-    }
-    return MARL_OK;
+// The step's buffers over B rows of X and T (n_rows: drawn from the first
+// n_rows of them; 0: taken in order).
+static mlp::TrainArgs train_args(marl_surrogate* s, uint32_t B, const __nv_bfloat16* X, const float* T,
+                                 uint32_t n_rows, float* loss_sum) {
+    mlp::TrainArgs a;
+    a.B = B, a.X = X, a.T = T, a.n_rows = n_rows, a.seed = s->cfg.seed, a.idx = s->idx;
+    a.w1 = s->w1, a.w2 = s->w2, a.w3 = s->w3, a.p = s->p;
+    a.h1 = s->h1, a.h2 = s->h2, a.dy = s->dy, a.dz2 = s->dz2, a.dz1 = s->dz1, a.d1 = s->d1, a.d2 = s->d2, a.y = s->y;
+    a.split_rows = mlp::train_split_rows(B), a.weight_part = s->weight_part, a.row_part = s->row_part;
+    a.g = s->g, a.loss_sum = loss_sum, a.err = s->d_err;
+    return a;
 }
 
 static marl_status check_err(marl_surrogate* s) {
@@ -240,9 +168,8 @@ marl_status marl_surrogate_config_default(marl_surrogate_config* c) {
 void marl_surrogate_destroy(marl_surrogate* s) {
     if (!s) return;
     if (s->stream) cudaStreamSynchronize(s->stream);
-    free_all({s->raw, s->X, s->T, s->norm, s->p, s->g, s->m, s->v, s->w1, s->w2, s->w3, s->w2t, s->w3t, s->xb,
-              s->xbt, s->h1, s->h1t, s->h2, s->h2t, s->dy, s->dyt, s->dz2, s->dz2t, s->dz1, s->dz1t, s->tb, s->z1,
-              s->z2, s->y, s->ih1, s->ih2, s->d_scalars, s->d_acc, s->d_err});
+    free_all({s->raw, s->X, s->T, s->norm, s->p, s->g, s->m, s->v, s->w1, s->w2, s->w3, s->xb, s->h1, s->h2, s->dy,
+              s->dz2, s->dz1, s->tb, s->d1, s->d2, s->y, s->idx, s->weight_part, s->row_part, s->ih1, s->ih2, s->d_scalars, s->d_acc, s->d_err});
     if (s->stream && s->own_stream) cudaStreamDestroy(s->stream);
     delete s;
 }
@@ -274,8 +201,6 @@ marl_status marl_surrogate_create(const marl_surrogate_config* cfg, marl_surroga
     if ((e = cudaMalloc((void**)&s->w1, (size_t)mlp::kHid * mlp::kInPad * 2)) ||
         (e = cudaMalloc((void**)&s->w2, (size_t)mlp::kHid * mlp::kHid * 2)) ||
         (e = cudaMalloc((void**)&s->w3, (size_t)mlp::kOut * mlp::kHid * 2)) ||
-        (e = cudaMalloc((void**)&s->w2t, (size_t)mlp::kHid * mlp::kHid * 2)) ||
-        (e = cudaMalloc((void**)&s->w3t, (size_t)mlp::kHid * mlp::kOutPad * 2)) ||
         (e = cudaMalloc((void**)&s->norm, MARL_SURR_NORM * 4)) || (e = cudaMalloc((void**)&s->d_acc, 256 * 8)) ||
         (e = cudaMalloc((void**)&s->d_err, 16)))
         return bad(e, "surrogate buffers");
@@ -283,7 +208,7 @@ marl_status marl_surrogate_create(const marl_surrogate_config* cfg, marl_surroga
     cudaMemsetAsync(s->v, 0, P * 4, s->stream);
     cudaMemsetAsync(s->d_err, 0, 16, s->stream);
     if ((e = mlp::launch_init_weights(s->p, cfg->seed, s->stream))) return bad(e, "init weights");
-    if ((e = mlp::launch_weights_bf16(s->p, s->w1, s->w2, s->w3, s->w2t, s->w3t, s->stream))) return bad(e, "bf16 weights");
+    if ((e = mlp::launch_weights_bf16(s->p, s->w1, s->w2, s->w3, s->stream))) return bad(e, "bf16 weights");
     if ((e = cudaStreamSynchronize(s->stream))) return bad(e, "surrogate create");
     *out = s;
     return MARL_OK;
@@ -375,15 +300,14 @@ marl_status marl_surrogate_train(marl_surrogate* s, uint32_t steps, float* loss_
     if (st) return st;
     if ((st = ensure_scalars(s, steps))) return st;
     cudaStream_t cs = s->stream;
-    SCK(cudaMemsetAsync(s->d_scalars, 0, (size_t)steps * 4, cs));
+    mlp::TrainArgs a = train_args(s, B, s->X, s->T, s->n_train, nullptr);
     for (uint32_t i = 0; i < steps; ++i) {
-        SCK(mlp::launch_gather_batch(s->X, s->T, s->n_train, s->cfg.seed, s->batches++, B, s->xb, s->xbt, s->tb, cs));
-        SST(forward_train(s, B));
-        SST(backward(s, B, s->d_scalars + i));
+        a.step = s->batches++;
+        a.loss_sum = s->d_scalars + i;
+        SCK(mlp::launch_forward_backward(a, cs));
         ++s->adam_t;
-        SCK(mlp::launch_adam(s->p, s->g, s->m, s->v, s->cfg.lr, s->cfg.beta1, s->cfg.beta2, s->cfg.adam_eps,
-                             s->adam_t, cs));
-        SCK(mlp::launch_weights_bf16(s->p, s->w1, s->w2, s->w3, s->w2t, s->w3t, cs));
+        SCK(mlp::launch_train_update(a, s->p, s->m, s->v, s->cfg.lr, s->cfg.beta1, s->cfg.beta2, s->cfg.adam_eps,
+                                     s->adam_t, s->w1, s->w2, s->w3, cs));
     }
     if (loss_out) {
         SCK(cudaMemcpyAsync(loss_out, s->d_scalars, (size_t)steps * 4, cudaMemcpyDeviceToHost, cs));
@@ -462,7 +386,7 @@ marl_status marl_surrogate_set_weights(marl_surrogate* s, const float* params, c
     // Ordered on the surrogate's stream, ahead of the kernels that read them.
     if (params) {
         SCK(cudaMemcpyAsync(s->p, params, (size_t)mlp::kParams * 4, cudaMemcpyHostToDevice, s->stream));
-        SCK(mlp::launch_weights_bf16(s->p, s->w1, s->w2, s->w3, s->w2t, s->w3t, s->stream));
+        SCK(mlp::launch_weights_bf16(s->p, s->w1, s->w2, s->w3, s->stream));
     }
     if (norm) {
         std::memcpy(s->h_norm, norm, sizeof(s->h_norm));
@@ -483,10 +407,9 @@ marl_status marl_surrogate_gradients(marl_surrogate* s, const uint16_t* x, const
     cudaStream_t cs = s->stream;
     SCK(cudaMemcpyAsync(s->xb, x, (size_t)batch * mlp::kInPad * 2, cudaMemcpyHostToDevice, cs));
     SCK(cudaMemcpyAsync(s->tb, t, (size_t)batch * mlp::kOut * 4, cudaMemcpyHostToDevice, cs));
-    SCK(mlp::launch_transpose_batch(s->xb, batch, s->xbt, cs));
-    SCK(cudaMemsetAsync(s->d_scalars, 0, 4, cs));
-    SST(forward_train(s, batch));
-    SST(backward(s, batch, s->d_scalars));
+    const mlp::TrainArgs a = train_args(s, batch, s->xb, s->tb, 0, s->d_scalars);
+    SCK(mlp::launch_forward_backward(a, cs));
+    SCK(mlp::launch_train_gradients(a, cs));
     SCK(cudaMemcpyAsync(grads_out, s->g, (size_t)mlp::kParams * 4, cudaMemcpyDeviceToHost, cs));
     float loss = 0.0f;
     SCK(cudaMemcpyAsync(&loss, s->d_scalars, 4, cudaMemcpyDeviceToHost, cs));

@@ -31,15 +31,16 @@ struct marl_surrogate {
     float* g = nullptr;  // gradients
     float* m = nullptr;  // Adam moments
     float* v = nullptr;
-    __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr, *w2t = nullptr, *w3t = nullptr;
+    __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr;
     uint64_t adam_t = 0;
     uint64_t batches = 0;  // batch counter (sampling stream)
 
     // Training work buffers for `work_b` rows.
     uint32_t work_b = 0;
-    __nv_bfloat16 *xb = nullptr, *xbt = nullptr, *h1 = nullptr, *h1t = nullptr, *h2 = nullptr, *h2t = nullptr;
-    __nv_bfloat16 *dy = nullptr, *dyt = nullptr, *dz2 = nullptr, *dz2t = nullptr, *dz1 = nullptr, *dz1t = nullptr;
-    float *tb = nullptr, *z1 = nullptr, *z2 = nullptr, *y = nullptr;
+    __nv_bfloat16 *xb = nullptr, *h1 = nullptr, *h2 = nullptr, *dy = nullptr, *dz2 = nullptr, *dz1 = nullptr;
+    float *tb = nullptr, *d1 = nullptr, *d2 = nullptr, *y = nullptr;  // xb, tb: a caller's batch (gradients)
+    uint32_t* idx = nullptr;
+    float *weight_part = nullptr, *row_part = nullptr;  // partial sums of the gradients and the loss
 
     // Inference work buffers for `infer_rows` rows.
     uint32_t infer_rows = 0;
