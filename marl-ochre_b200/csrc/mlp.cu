@@ -110,7 +110,8 @@ __global__ void __launch_bounds__(kGemmThreads) k_gemm(const __grid_constant__ G
         if constexpr (EPI == EPI_BIAS_GELU_FAST) {
             float h[16];
 #pragma unroll
-            for (int i = 0; i < 16; ++i) h[i] = gelu_fast(v[i] + a.bias[n + i]);
+            for (int i = 0; i < 16; i += 2)
+                gelu_fast2(pair_f32(v[i], v[i + 1]), pair_f32(a.bias[n + i], a.bias[n + i + 1]), h[i], h[i + 1]);
             if (row_ok) {
                 uint4* o = reinterpret_cast<uint4*>(a.out_bf + (size_t)row * a.ldo + n);
                 o[0] = make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]),
@@ -157,19 +158,30 @@ cudaError_t launch_gemm(const GemmArgs& a, int bn, int epi, cudaStream_t s) {
 }
 
 // ------------------------------------------------------- fused inference --
-// The whole forward pass in one persistent kernel: one CTA per SM (8 warps)
+// The whole forward pass in one persistent kernel: one CTA per SM (16 warps)
 // walks 128-row tiles.  All weights stay in shared memory for the kernel's
 // life (W1 256 x 128, W2 256 x 256, W3 16 x 256: 200 KB, 128B-swizzled).  The
 // activations never leave the SM: a tile's inputs and hidden layers live in
 // tensor memory as BF16 and feed the next MMA as its A operand straight from
 // tensor memory (the TS form of tcgen05.mma; A is row-per-lane, two BF16 per
 // 32-bit column, lower k in the low half).  Tensor-memory columns: 0-255 the
-// FP32 accumulator of layers 1 and 2, 256-383 the hidden layer (BF16),
-// 384-447 the inputs (BF16), 448-463 the accumulator of layer 3.  Warp w owns
-// TMEM lanes 32(w%4).. (tile rows) and column half w/4 in the epilogues.  The
+// FP32 accumulator of layers 1 and 2, 256-383 the first hidden layer (BF16),
+// 384-447 the inputs (BF16), 448-463 the accumulator of layer 3; the second
+// hidden layer overwrites the accumulator it comes from, each warp its own 64
+// columns (once it has read them all).
+//
+// What bounds it: 512 hardware tanh a row, 34 us for 300,000 rows on the MUFU
+// pipes, against 26 us of tensor-core time.  Each hidden layer is two MMAs of
+// 128 columns with a commit each, and two groups of eight warps: while a group
+// takes the activations of the first half, the tensor core works on the
+// second.  Warp w owns TMEM lanes 32 (w % 4).. (tile rows) and 64 columns, read
+// in two 32-column loads that are both in flight before the first is used.  The
 // next tile's inputs are read from global memory into registers during
-// epilogue 1 and stored to tensor memory while layer 2 runs.
-constexpr int kFusedThreads = 256;
+// epilogue 1 and stored to tensor memory while layer 2 runs; its layer 1 is
+// issued before the output of this tile is written.
+// 300,000 rows: 144 us with one 256-column MMA a layer, 8 warps and scalar
+// activation arithmetic.
+constexpr int kFusedThreads = 512;
 constexpr uint32_t kFW1 = kHid * kInPad * 2;   // 64 KB
 constexpr uint32_t kFW2 = kHid * kHid * 2;     // 128 KB
 constexpr uint32_t kFW3 = kOut * kHid * 2;     // 8 KB
@@ -207,55 +219,52 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// Row `row` of the inputs, K half `half` (64 BF16 = 32 TMEM columns), read
+// Row `row` of the inputs, K quarter `part` (32 BF16 = 16 TMEM columns), read
 // into registers; zeros beyond M.
-__device__ __forceinline__ void load_x_half(const __nv_bfloat16* x, int M, int row, int half, uint32_t (&r)[32]) {
+__device__ __forceinline__ void load_x_part(const __nv_bfloat16* x, int M, int row, int part, uint32_t (&r)[16]) {
     if (row < M) {
-        const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * kInPad + half * 64);
+        const uint4* src = reinterpret_cast<const uint4*>(x + (size_t)row * kInPad + part * 32);
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
+        for (int i = 0; i < 4; ++i) {
             const uint4 v = __ldg(src + i);
             r[4 * i] = v.x, r[4 * i + 1] = v.y, r[4 * i + 2] = v.z, r[4 * i + 3] = v.w;
         }
     } else {
 #pragma unroll
-        for (int i = 0; i < 32; ++i) r[i] = 0u;
+        for (int i = 0; i < 16; ++i) r[i] = 0u;
     }
 }
 
-__device__ __forceinline__ void store_x_half(uint32_t t_lane, int half, const uint32_t (&r)[32]) {
-    uint32_t lo[16], hi[16];
+// Epilogue of a hidden layer: 64 columns of the accumulator from `from` ->
+// gelu(acc + bias) -> 32 columns of BF16 pairs at `to` (which may be the same
+// columns: all are read first).  `bias` is in shared memory, 16-byte aligned.
+__device__ __forceinline__ void hidden_epilogue(uint32_t from, uint32_t to, const float* bias) {
+    uint32_t r[2][32];
+    tmem_ld32_issue(from, r[0]);
+    tmem_ld32_issue(from + 32, r[1]);
+    tmem_ld_wait();
 #pragma unroll
-    for (int i = 0; i < 16; ++i) lo[i] = r[i], hi[i] = r[16 + i];
-    tmem_st16(t_lane + kTX + half * 32, lo);
-    tmem_st16(t_lane + kTX + half * 32 + 16, hi);
-}
-
-// Epilogue of a hidden layer: columns [half*128, +128) of the accumulator ->
-// gelu(acc + bias) -> BF16 pairs into the hidden-layer columns.
-__device__ __forceinline__ void hidden_epilogue(uint32_t t_lane, int half, const float* bias) {
-#pragma unroll 1
-    for (int cb = 0; cb < 128; cb += 32) {
-        const int n = half * 128 + cb;
-        float v[16], u[16];
-        tmem_ld16(t_lane + kTAcc + n, v);
-        tmem_ld16(t_lane + kTAcc + n + 16, u);
+    for (int b = 0; b < 2; ++b) {
         uint32_t w[16];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            w[i] = pack_bf16(gelu_fast(v[2 * i] + bias[n + 2 * i]), gelu_fast(v[2 * i + 1] + bias[n + 2 * i + 1]));
-            w[8 + i] = pack_bf16(gelu_fast(u[2 * i] + bias[n + 16 + 2 * i]),
-                                 gelu_fast(u[2 * i + 1] + bias[n + 16 + 2 * i + 1]));
+            const float4 bb = reinterpret_cast<const float4*>(bias)[8 * b + i];
+            const uint32_t* v = &r[b][4 * i];
+            float h0, h1, h2, h3;
+            gelu_fast2(pair_f32(__uint_as_float(v[0]), __uint_as_float(v[1])), pair_f32(bb.x, bb.y), h0, h1);
+            gelu_fast2(pair_f32(__uint_as_float(v[2]), __uint_as_float(v[3])), pair_f32(bb.z, bb.w), h2, h3);
+            w[2 * i] = pack_bf16(h0, h1);
+            w[2 * i + 1] = pack_bf16(h2, h3);
         }
-        tmem_st16(t_lane + kTH + n / 2, w);
+        tmem_st16(to + 16 * b, w);
     }
 }
 
 __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs a) {
     extern __shared__ uint8_t fsm_raw[];
-    __shared__ uint64_t bars[3];  // one per layer
+    __shared__ uint64_t bars[5];  // layer 1 halves, layer 2 halves, layer 3
     __shared__ uint32_t tmem_slot;
-    __shared__ float sb1[kHid], sb2[kHid], sb3[kOut], sscale[kOut], sshift[kOut];
+    __shared__ __align__(16) float sb1[kHid], sb2[kHid], sb3[kOut], sscale[kOut], sshift[kOut];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t base = (smem_u32(fsm_raw) + 1023u) & ~1023u;
     const uint32_t sW1 = base, sW2 = sW1 + kFW1, sW3 = sW2 + kFW2;
@@ -267,7 +276,7 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs a) {
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        for (int i = 0; i < 3; ++i) mbar_init(&bars[i], 1);
+        for (int i = 0; i < 5; ++i) mbar_init(&bars[i], 1);
         fence_mbar_init();
     }
     load_sw128(sW1, a.w1, kInPad, kHid, kInPad, tid, kFusedThreads);
@@ -275,78 +284,88 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs a) {
     load_sw128(sW3, a.w3, kHid, kOut, kHid, tid, kFusedThreads);
     for (int i = tid; i < kHid; i += kFusedThreads) sb1[i] = a.b1[i], sb2[i] = a.b2[i];
     if (tid < kOut) sb3[tid] = a.b3[tid], sscale[tid] = a.scale[tid], sshift[tid] = a.shift[tid];
+    const int quarter = warp & 3, part = warp >> 2;  // tile rows; columns 64 part .. 64 part + 63
+    const int half = part >> 1;
+    const int ntiles = (a.M + kBM - 1) / kBM;
+    int tile = blockIdx.x;
+    uint32_t xr[16];
+    load_x_part(a.x, a.M, tile * kBM + quarter * 32 + lane, part, xr);
     cp_async_commit_wait_all();
     fence_proxy_async_smem();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_slot;
-    const int quarter = warp & 3, half = warp >> 2;
     const uint32_t t_lane = tmem + ((uint32_t)(quarter * 32) << 16);
-    const int ntiles = (a.M + kBM - 1) / kBM;
+    constexpr uint32_t idesc = idesc_bf16(kBM, kHid / 2);
+    // One half of a hidden layer: columns [128 h, +128) of the accumulator.
+    auto layer1 = [&](int h) {
+#pragma unroll
+        for (int k = 0; k < kInPad / 16; ++k)
+            umma_bf16_ts(tmem + kTAcc + h * 128, tmem + kTX + k * 8,
+                         sw128_desc(sW1 + (k >> 2) * kHid * 128 + h * 128 * 128 + (k & 3) * 32), idesc, k > 0 ? 1u : 0u);
+        umma_commit(&bars[h]);
+    };
+    auto layer2 = [&](int h) {
+#pragma unroll
+        for (int k = 0; k < kHid / 16; ++k)
+            umma_bf16_ts(tmem + kTAcc + h * 128, tmem + kTH + k * 8,
+                         sw128_desc(sW2 + (k >> 2) * kHid * 128 + h * 128 * 128 + (k & 3) * 32), idesc, k > 0 ? 1u : 0u);
+        umma_commit(&bars[2 + h]);
+    };
     bool ok = true;
     uint32_t it = 0;
-    uint32_t xr[32];
-    int tile = blockIdx.x;
-    if (tile < ntiles) {
-        load_x_half(a.x, a.M, tile * kBM + quarter * 32 + lane, half, xr);
-        store_x_half(t_lane, half, xr);
-        tmem_st_wait();
-    }
+    tmem_st16(t_lane + kTX + part * 16, xr);
+    tmem_st_wait();
     tc_fence_before();
     __syncthreads();
+    if (tid == 0) {
+        tc_fence_after();
+        layer1(0);
+        layer1(1);
+    }
 
     for (; tile < ntiles; tile += gridDim.x, ++it) {
-        const int m0 = tile * kBM;
-        // layer 1: acc = X W1^T (A = inputs in tensor memory)
-        if (tid == 0) {
-            tc_fence_after();
-#pragma unroll
-            for (int k = 0; k < kInPad / 16; ++k)
-                umma_bf16_ts(tmem + kTAcc, tmem + kTX + k * 8,
-                             sw128_desc(sW1 + (k >> 2) * kHid * 128 + (k & 3) * 32), idesc_bf16(kBM, kHid),
-                             k > 0 ? 1u : 0u);
-            umma_commit(&bars[0]);
-        }
-        ok = wait_commit(&bars[0], it & 1, a.err) && ok;
+        const int m0 = tile * kBM, next = tile + gridDim.x;
+        ok = wait_commit(&bars[half], it & 1, a.err) && ok;
         tc_fence_after();
-        const int next = tile + gridDim.x;
-        if (next < ntiles) load_x_half(a.x, a.M, next * kBM + quarter * 32 + lane, half, xr);  // in flight
-        hidden_epilogue(t_lane, half, sb1);
+        if (next < ntiles) load_x_part(a.x, a.M, next * kBM + quarter * 32 + lane, part, xr);  // in flight
+        hidden_epilogue(t_lane + kTAcc + part * 64, t_lane + kTH + part * 32, sb1 + part * 64);
         tmem_st_wait();
         tc_fence_before();
         __syncthreads();
-        // layer 2: acc = H W2^T (A = hidden layer in tensor memory)
+        if (tid == 0) {
+            tc_fence_after();
+            layer2(0);
+            layer2(1);
+        }
+        // The next tile's inputs go to tensor memory while layer 2 runs (both
+        // halves of layer 1 are done with them: every warp has seen its own).
+        if (next < ntiles) tmem_st16(t_lane + kTX + part * 16, xr);
+        ok = wait_commit(&bars[2 + half], it & 1, a.err) && ok;
+        tc_fence_after();
+        hidden_epilogue(t_lane + kTAcc + part * 64, t_lane + kTAcc + part * 64, sb2 + part * 64);
+        tmem_st_wait();
+        tc_fence_before();
+        __syncthreads();
         if (tid == 0) {
             tc_fence_after();
 #pragma unroll
             for (int k = 0; k < kHid / 16; ++k)
-                umma_bf16_ts(tmem + kTAcc, tmem + kTH + k * 8,
-                             sw128_desc(sW2 + (k >> 2) * kHid * 128 + (k & 3) * 32), idesc_bf16(kBM, kHid),
-                             k > 0 ? 1u : 0u);
-            umma_commit(&bars[1]);
-        }
-        // the next tile's inputs go to tensor memory while layer 2 runs (layer 1 is done with them)
-        if (next < ntiles) store_x_half(t_lane, half, xr);
-        ok = wait_commit(&bars[1], it & 1, a.err) && ok;
-        tc_fence_after();
-        hidden_epilogue(t_lane, half, sb2);
-        tmem_st_wait();
-        tc_fence_before();
-        __syncthreads();
-        // layer 3: acc3 = H W3^T
-        if (tid == 0) {
-            tc_fence_after();
-#pragma unroll
-            for (int k = 0; k < kHid / 16; ++k)
-                umma_bf16_ts(tmem + kTAcc3, tmem + kTH + k * 8,
+                umma_bf16_ts(tmem + kTAcc3, tmem + kTAcc + (k >> 2) * 64 + (k & 3) * 8,
                              sw128_desc(sW3 + (k >> 2) * kOut * 128 + (k & 3) * 32), idesc_bf16(kBM, kOut),
                              k > 0 ? 1u : 0u);
-            umma_commit(&bars[2]);
+            umma_commit(&bars[4]);
         }
-        ok = wait_commit(&bars[2], it & 1, a.err) && ok;
+        ok = wait_commit(&bars[4], it & 1, a.err) && ok;
         tc_fence_after();
-        if (half == 0) {
+        // Layer 3 is done with the hidden layer in the accumulator's columns, and
+        // the next tile's inputs were stored before the barrier above.
+        if (tid == 0 && next < ntiles) {
+            layer1(0);
+            layer1(1);
+        }
+        if (part == 3) {  // not the warp that issues
             float v[16];
             tmem_ld16(t_lane + kTAcc3, v);
             const int row = m0 + quarter * 32 + lane;
@@ -356,10 +375,10 @@ __global__ void __launch_bounds__(kFusedThreads, 1) k_mlp_fused(FusedArgs a) {
                     a.y[(size_t)i * a.ldy + row] = (v[i] + sb3[i]) * sscale[i] + sshift[i];
             }
         }
-        tc_fence_before();
-        __syncthreads();
+        // The accumulator of layer 3 is read before the barriers of the next
+        // tile, and so before it is written again.
     }
-    tc_fence_after();
+    tc_fence_before();
     __syncthreads();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");

@@ -69,6 +69,19 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
+// 32 columns of the warp's lanes, without waiting (tmem_ld_wait).
+__device__ __forceinline__ void tmem_ld32_issue(uint32_t taddr, uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,%17,%18,"
+        "%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
+        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
+          "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]),
+          "=r"(r[16]), "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]),
+          "=r"(r[24]), "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
+        : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld_wait() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
     uint32_t r[16];
     asm volatile(
@@ -89,12 +102,41 @@ __device__ __forceinline__ float gelu_and_grad(float z, float& grad) {
     return 0.5f * z * (1.0f + t);
 }
 // Inference form: the hardware tanh approximation (MUFU), max relative error
-// about 2^-11, below the BF16 rounding the activation goes through next.
-__device__ __forceinline__ float gelu_fast(float z) {
-    const float u = 0.7978845608028654f * (z + 0.044715f * z * z * z);
-    float t;
-    asm("tanh.approx.f32 %0, %1;" : "=f"(t) : "f"(u));
-    return 0.5f * z * (1.0f + t);
+// about 2^-11, below the BF16 rounding the activation goes through next.  Two
+// values at a time, two to a packed FP32 operation (each half is the scalar
+// round-to-nearest operation): 8 packed operations and two MUFU a pair, so the
+// MUFU pipe (16 a cycle and SM) is what bounds an epilogue.
+__device__ __forceinline__ uint64_t pair_f32(float a, float b) {
+    uint64_t r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+    uint64_t r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+    uint64_t r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ void gelu_fast2(uint64_t acc, uint64_t bias, float& h0, float& h1) {
+    // z = acc + bias; u = sqrt(2/pi) (z + 0.044715 z z z); h = z / 2 (1 + tanh u)
+    const uint64_t z = add2(acc, bias);
+    const uint64_t zz = mul2(mul2(pair_f32(0.044715f, 0.044715f), z), z);
+    const uint64_t u = mul2(pair_f32(0.7978845608028654f, 0.7978845608028654f), fma2(zz, z, z));
+    float u0, u1, t0, t1;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(u0), "=f"(u1) : "l"(u));
+    asm("tanh.approx.f32 %0, %1;" : "=f"(t0) : "f"(u0));
+    asm("tanh.approx.f32 %0, %1;" : "=f"(t1) : "f"(u1));
+    const uint64_t h = mul2(mul2(pair_f32(0.5f, 0.5f), z), add2(pair_f32(1.0f, 1.0f), pair_f32(t0, t1)));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(h0), "=f"(h1) : "l"(h));
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
