@@ -1312,8 +1312,8 @@ static cudaError_t launch_cell_tick_quad(const CellLaunch& a, int num_sms, cudaS
     int per_sm = 1;
     cudaError_t e = quad_per_sm(setup, k_cell_tick_quad, &per_sm);
     if (e != cudaSuccess) return e;
-    // Persistent: never more blocks than can be resident at once.
-    const uint32_t needed = blocks_for(a.n, kQuadCells), resident = (uint32_t)per_sm * (uint32_t)num_sms;
+    // Persistent: never more blocks than can be resident at once, down to a cell a warp.
+    const uint32_t needed = blocks_for(a.n, kQuadThreads / 32), resident = (uint32_t)per_sm * (uint32_t)num_sms;
     k_cell_tick_quad<<<needed < resident ? needed : resident, kQuadThreads, kQuadSmem, s>>>(a);
     return cudaGetLastError();
 }
@@ -1470,7 +1470,7 @@ cudaError_t launch_cell_tick_batch(const RunDesc* runs, int n_runs, BatchScalars
             int per_sm = 1;
             cudaError_t e = quad_per_sm(setup, k_cell_tick_quad_batch, &per_sm);
             if (e != cudaSuccess) return e;
-            const uint64_t needed = (total_cap + kQuadCells - 1) / kQuadCells, resident = (uint64_t)per_sm * num_sms;
+            const uint64_t needed = (total_cap + kQuadThreads / 32 - 1) / (kQuadThreads / 32), resident = (uint64_t)per_sm * num_sms;
             CellConsts here = k;
             here.schedule_here = 1;
             k_cell_tick_quad_batch<<<(unsigned)(needed < resident ? needed : resident), kQuadThreads, kQuadSmem, s>>>(

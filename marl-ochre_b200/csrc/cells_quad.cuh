@@ -95,10 +95,10 @@ struct __align__(16) QuadCell {
     float ext[MARL_S_EXT];
     float del[MARL_S_EXT];
     uint32_t pos, state, age, nb;
-    int32_t dep[6];
+    int32_t dep[6];  // dependencies by face; after the plan the different ones, then -1
     uint32_t info;  // reactions that run | transporter rounds << 8 | effector rounds << 16 | flags
     uint32_t rounds[4];  // lane p's slots, a byte each: transporters p, p + 4, effectors p, p + 4 (kQuadOut: left out)
-    uint32_t pad;
+    uint32_t vox;  // the cell's voxel
     float2 secretion[4];  // lane p's transporters' secretion where their round is 0: nothing changes their species before
     QuadAt at;  // batch only
 };
@@ -261,6 +261,16 @@ __device__ __forceinline__ uint32_t quad_rounds(const uint4& w, uint32_t part, i
     return rounds;
 }
 
+// Face f's voxel from the voxel at `at` (spatial.rs:8-15).
+__device__ __forceinline__ float* quad_face(float* at, int X, int Y, int f) {
+    const uint32_t row = (uint32_t)X * 12, slab = (uint32_t)Y * row;
+    const size_t off = f < 2 ? 12u : (f < 4 ? row : slab);
+    return f & 1 ? at - off : at + off;
+}
+__device__ __forceinline__ size_t quad_voxel(int X, int Y, uint32_t P) {
+    return ((size_t)pos_z(P) * Y + pos_y(P)) * X + pos_x(P);
+}
+
 // Derives the plan of a staged cell (groups with `fresh`; the whole warp takes
 // part, other groups compute on what lies in their record and store nothing).
 //
@@ -274,7 +284,26 @@ __device__ __forceinline__ uint32_t quad_rounds(const uint4& w, uint32_t part, i
 //   - dt, epsilon and c_max are ordinary numbers.
 // kQuadPlain says that all of this holds but for the gathered values and the
 // light, which the update checks.
-__device__ __forceinline__ void quad_plan(const CellConsts& c, QuadCell& C, int p, bool fresh) {
+__device__ __forceinline__ void quad_plan(const CellConsts& c, QuadCell& C, int p, bool fresh, int X, int Y) {
+    // Lane p waits for the p-th and the (p + 4)-th different dependency: more
+    // than four are rare, and a lane's two acquire loads follow one another.
+    int32_t wait[2] = {-1, -1};
+    {
+        int32_t d[6];
+        int found = 0;
+#pragma unroll
+        for (int f = 0; f < 6; ++f) {
+            d[f] = C.dep[f];
+            bool is_new = d[f] >= 0;
+#pragma unroll
+            for (int e = 0; e < f; ++e) is_new = is_new && d[e] != d[f];
+            if (is_new) {
+                if (found == p) wait[0] = d[f];
+                if (found == p + 4) wait[1] = d[f];
+                ++found;
+            }
+        }
+    }
     const float inf = __uint_as_float(0x7F800000u);
     bool plain = c.dt >= 0.0f && c.dt < inf && c.epsilon >= 0.0f && c.epsilon < kQuadRateMax && c.c_max > 0.0f &&
                  c.c_max <= kQuadValueMax;
@@ -352,10 +381,13 @@ __device__ __forceinline__ void quad_plan(const CellConsts& c, QuadCell& C, int 
     plain = group_ballot(plain) == 0xFu;
     cof = group_ballot(cof) != 0;
     if (fresh) {
+        C.dep[p] = wait[0];
+        if (p < 2) C.dep[p + 4] = wait[1];
         C.rounds[p] = to[0] | to[1] << 8 | eo[0] << 16 | eo[1] << 24;
         C.secretion[p] = make_float2(sec[0], sec[1]);
         if (p == 0) {
             C.x[kQuadZero] = 0.0f;
+            C.vox = (uint32_t)quad_voxel(X, Y, C.pos);
             C.keep = keep;
             C.cost = cost;
             C.info = __popc(run) | nt << 8 | ne << 16 | (plain ? kQuadPlain : 0u) | (cof ? kQuadCofactor : 0u);
@@ -394,16 +426,6 @@ __device__ __forceinline__ void quad_fate(const CellConsts& c, const QuadAt& t, 
     t.age[t.j] = C.age + 1;
     t.state[t.j] = (st & 0xFF000000u) | (quiescent << 16) | prep;
     t.events[t.j] = event;
-}
-
-// Face f's voxel from the voxel at `at` (spatial.rs:8-15).
-__device__ __forceinline__ float* quad_face(float* at, int X, int Y, int f) {
-    const uint32_t row = (uint32_t)X * 12, slab = (uint32_t)Y * row;
-    const size_t off = f < 2 ? 12u : (f < 4 ? row : slab);
-    return f & 1 ? at - off : at + off;
-}
-__device__ __forceinline__ size_t quad_voxel(int X, int Y, uint32_t P) {
-    return ((size_t)pos_z(P) * Y + pos_y(P)) * X + pos_x(P);
 }
 
 // The whole update of cell j by one lane, for any values.
@@ -645,7 +667,7 @@ template <class View>
 __device__ __forceinline__ bool quad_update(const View& v, const CellConsts& c, QuadCell& C, int p, bool ready) {
     const uint32_t nb = ready ? C.nb : 0u;
     const int n = __popc(nb);
-    const size_t vox = ready ? quad_voxel(v.X(), v.Y(), C.pos) : 0;
+    const size_t vox = ready ? C.vox : 0u;
     float* const at = v.field() + vox * 12 + 4 * p;
 
     // Gather (spatial.rs:56-77), summed in face order from 0.0; a face that is
@@ -717,6 +739,11 @@ __device__ __forceinline__ void quad_loop(QuadCell* cells, const CellConsts& c, 
                                           uint32_t* err, Stage stage, Look look) {
     const unsigned FULL = 0xFFFFFFFFu;
     const int lane = threadIdx.x & 31, p = lane & 3;
+    // Cells a warp holds: as few as the grid's warps need to hold all of them,
+    // so that they wait on one another's passes as little as possible.
+    const uint32_t warps = gridDim.x * (kQuadThreads / 32), per_warp = min((total + warps - 1) / warps, 8u);
+    if ((blockIdx.x * (kQuadThreads / 32) + (threadIdx.x >> 5)) * per_warp >= total) return;  // earlier warps hold them
+    const bool usable = (uint32_t)(lane >> 2) < per_warp;
     QuadCell& C = cells[threadIdx.x >> 2];
     bool pending = false, fresh = false, more = true;
     uint32_t gi = 0, waiting = 0, spins = 0;
@@ -724,7 +751,8 @@ __device__ __forceinline__ void quad_loop(QuadCell* cells, const CellConsts& c, 
         if (__any_sync(FULL, fresh)) {
             cp_async_wait_all();
             __syncwarp();
-            quad_plan(c, C, p, fresh);
+            const auto w = look(C, gi);
+            quad_plan(c, C, p, fresh, w.X(), w.Y());
             if (fresh) {
                 waiting = (pending && C.dep[p] >= 0 ? 1u : 0u) | (pending && p < 2 && C.dep[p + 4] >= 0 ? 2u : 0u);
                 fresh = false;
@@ -740,7 +768,7 @@ __device__ __forceinline__ void quad_loop(QuadCell* cells, const CellConsts& c, 
         }
         ready = group_ballot(ready) == 0xFu;
         const unsigned run = __ballot_sync(FULL, ready);
-        const unsigned free_lanes = __ballot_sync(FULL, !pending || ready);
+        const unsigned free_lanes = __ballot_sync(FULL, usable && (!pending || ready));
         uint32_t base = 0;
         if (more && free_lanes && lane == 0) base = atomicAdd(ticket, (uint32_t)__popc(free_lanes) >> 2);
         if (run) {  // an update publishes its cell itself
@@ -786,7 +814,6 @@ __global__ void __launch_bounds__(kQuadThreads, kQuadBlocksPerSM)
     extern __shared__ __align__(16) unsigned char tick_smem[];
     const uint32_t total = a.n_dev ? *a.n_dev : a.n;
     if (a.split && total > a.split) return;
-    if (blockIdx.x * kQuadCells >= total) return;  // the earlier blocks' groups hold every cell at once
     quad_loop(
         reinterpret_cast<QuadCell*>(tick_smem), a.k, total, a.ticket, a.err,
         [&](QuadCell& C, uint32_t gi, int p) {
@@ -802,7 +829,6 @@ __global__ void __launch_bounds__(kQuadThreads, kQuadBlocksPerSM)
     extern __shared__ __align__(16) unsigned char tick_smem[];
     const uint32_t total = batch_total(runs, n_runs);
     if (total > split) return;
-    if (blockIdx.x * kQuadCells >= total) return;  // the earlier blocks' groups hold every cell at once
     quad_loop(
         reinterpret_cast<QuadCell*>(tick_smem), c, total, &bs->ticket, &bs->err,
         [&](QuadCell& C, uint32_t gi, int p) {
