@@ -1016,35 +1016,44 @@ marl_status marl_diffuse_device(float* field_dev, float* scratch_dev, const uint
     FieldConsts fk;
     CellConsts ck;
     derive_consts(*sim, &fk, &ck);
-    // Workspace: the error word, then the padded mask where the caller's rows
-    // cannot be read in place.
-    const bool in_place = mask_in_place(occ_dev, g);
+    ResidentPlan rp;
+    const bool resident = resident_plan(g, substeps, sms, &rp);
+    // Workspace: the error word, then the resident kernel's mailboxes or the
+    // padded mask where the caller's rows cannot be read in place.
+    constexpr size_t head = 256;
+    const size_t mail = resident ? resident_mail_bytes(rp) : 0;
+    const bool in_place = resident || mask_in_place(occ_dev, g);
     uint8_t* work = nullptr;
-    CK(work_alloc(&work, 256 + (in_place ? 0 : (size_t)gz * gy * mask_pitch(gx)), dev, s));
+    CK(work_alloc(&work, head + mail + (in_place ? 0 : (size_t)gz * gy * mask_pitch(gx)), dev, s));
     uint32_t* err = reinterpret_cast<uint32_t*>(work);
-    cudaError_t e = cudaMemsetAsync(err, 0, 4, s);
+    cudaError_t e = cudaMemsetAsync(work, 0, resident ? head + mail : 4, s);
     const uint8_t* mask = occ_dev;
     if (!in_place) {
-        mask = work + 256;
-        if (e == cudaSuccess) e = launch_repack_mask(occ_dev, work + 256, g, s);
+        mask = work + head;
+        if (e == cudaSuccess) e = launch_repack_mask(occ_dev, work + head, g, s);
     }
     auto bail = [&](marl_status st) {
         cudaFreeAsync(work, s);
         return st;
     };
     if (e != cudaSuccess) return bail(cuda_fail(e, "occupancy mask"));
-    DiffusionPlan plan;
-    int tile, zc;
-    default_diffusion_tile(&g, 1, sms, &tile, &zc);
-    if (!plan_diffusion(&plan, field_dev, scratch_dev, mask, g, tile, zc))
-        return bail(fail(MARL_ERR_CUDA, "cuTensorMapEncodeTiled failed"));
-    int cur = 0;  // 0: field_dev holds the live state, 1: scratch_dev does
-    for (uint32_t i = 0; i < substeps && e == cudaSuccess; ++i) {
-        e = launch_diffuse(plan, cur, g, fk, 0, nullptr, err, s);
-        cur ^= 1;
+    if (resident) {
+        e = launch_diffuse_resident(rp, field_dev, occ_dev, gx, g, fk, (int)substeps, 0, nullptr, work + head, 0, err,
+                                    s);
+    } else {
+        DiffusionPlan plan;
+        int tile, zc;
+        default_diffusion_tile(&g, 1, sms, &tile, &zc);
+        if (!plan_diffusion(&plan, field_dev, scratch_dev, mask, g, tile, zc))
+            return bail(fail(MARL_ERR_CUDA, "cuTensorMapEncodeTiled failed"));
+        int cur = 0;  // 0: field_dev holds the live state, 1: scratch_dev does
+        for (uint32_t i = 0; i < substeps && e == cudaSuccess; ++i) {
+            e = launch_diffuse(plan, cur, g, fk, 0, nullptr, err, s);
+            cur ^= 1;
+        }
+        if (cur != 0 && e == cudaSuccess)
+            e = cudaMemcpyAsync(field_dev, scratch_dev, g.V() * 48, cudaMemcpyDeviceToDevice, s);
     }
-    if (cur != 0 && e == cudaSuccess)
-        e = cudaMemcpyAsync(field_dev, scratch_dev, g.V() * 48, cudaMemcpyDeviceToDevice, s);
     uint32_t h_err = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h_err, err, 4, cudaMemcpyDeviceToHost, s);
     if (e != cudaSuccess) return bail(cuda_fail(e, "diffusion substeps"));

@@ -14,6 +14,8 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "internal.h"
 #include "kernel_setup.h"
@@ -477,6 +479,8 @@ __global__ void __launch_bounds__(kDiffTX* TY, (diff_min_blocks<TY, DIRECT>()))
     diffuse_tile<TY, STAGES, DIRECT>(&m[parity], &m[2 + (parity ^ 1)], &m[4], r.g, it.y, it.z, it.w, zc, k,
                                      apply_sources, emit_c4 ? r.c4 : nullptr, err, r.field[parity ^ 1]);
 }
+
+#include "field_resident.cuh"
 
 // ------------------------------------------------------------ light ------
 // crates/marl-field/src/light.rs:29-59.  The running intensity of a column is

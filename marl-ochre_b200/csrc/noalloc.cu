@@ -12,7 +12,8 @@
 //
 // Scratch: one array, g_noalloc_scratch, holding (1) the ping-pong copy of the
 // field, (2) the occupancy mask with rows padded to 16 bytes (the TMA stride
-// rule), (3) the error word.  Limits: at most kNoAllocMaxVoxels voxels, and
+// rule), (3) the error word.  The kernel for small grids keeps its mailboxes in
+// (1).  Limits: at most kNoAllocMaxVoxels voxels, and
 // Y * Z * (X rounded up to 16) <= kNoAllocMaskBytes.  Every GPU that loads the
 // library holds the array (about 13 MiB) until the process exits.
 //
@@ -94,22 +95,32 @@ extern "C" marl_status marl_diffuse_device_noalloc(float* field_dev, const uint8
     derive_consts(*sim, &fk, &ck);
     cudaError_t e = cudaMemsetAsync(err, 0, 4, s);
     if (e != cudaSuccess) return cuda_fail(e, "clear error word");
-    const bool in_place = mask_in_place(occupancy_dev, g);
-    if (!in_place && (e = launch_repack_mask(occupancy_dev, mask, g, s)) != cudaSuccess)
-        return cuda_fail(e, "repack occupancy");
-    DiffusionPlan plan;
-    int tile, zc;
-    default_diffusion_tile(&g, 1, sms, &tile, &zc);
-    if (!plan_diffusion(&plan, field_dev, scratch, in_place ? occupancy_dev : mask, g, tile, zc))
-        return fail(MARL_ERR_CUDA, "cuTensorMapEncodeTiled failed");
-    int cur = 0;  // 0: field_dev holds the live state, 1: the scratch copy does
-    for (uint32_t i = 0; i < substeps; ++i) {
-        if ((e = launch_diffuse(plan, cur, g, fk, 0, nullptr, err, s)) != cudaSuccess)
-            return cuda_fail(e, "diffusion substep");
-        cur ^= 1;
+    ResidentPlan rp;
+    if (resident_plan(g, substeps, sms, &rp) && resident_mail_bytes(rp) <= kNoAllocFieldBytes) {
+        // The kernel's mailboxes in place of the ping-pong copy, which it has no use for.
+        if ((e = cudaMemsetAsync(scratch, 0, resident_mail_bytes(rp), s)) == cudaSuccess)
+            e = launch_diffuse_resident(rp, field_dev, occupancy_dev, gx, g, fk, (int)substeps, 0, nullptr, scratch, 0,
+                                        err, s);
+        if (e != cudaSuccess) return cuda_fail(e, "diffusion substeps");
+    } else {
+        const bool in_place = mask_in_place(occupancy_dev, g);
+        if (!in_place && (e = launch_repack_mask(occupancy_dev, mask, g, s)) != cudaSuccess)
+            return cuda_fail(e, "repack occupancy");
+        DiffusionPlan plan;
+        int tile, zc;
+        default_diffusion_tile(&g, 1, sms, &tile, &zc);
+        if (!plan_diffusion(&plan, field_dev, scratch, in_place ? occupancy_dev : mask, g, tile, zc))
+            return fail(MARL_ERR_CUDA, "cuTensorMapEncodeTiled failed");
+        int cur = 0;  // 0: field_dev holds the live state, 1: the scratch copy does
+        for (uint32_t i = 0; i < substeps; ++i) {
+            if ((e = launch_diffuse(plan, cur, g, fk, 0, nullptr, err, s)) != cudaSuccess)
+                return cuda_fail(e, "diffusion substep");
+            cur ^= 1;
+        }
+        if (cur != 0 &&
+            (e = cudaMemcpyAsync(field_dev, scratch, g.V() * 48, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
+            return cuda_fail(e, "copy result");
     }
-    if (cur != 0 && (e = cudaMemcpyAsync(field_dev, scratch, g.V() * 48, cudaMemcpyDeviceToDevice, s)) != cudaSuccess)
-        return cuda_fail(e, "copy result");
     uint32_t h_err = 0;
     if ((e = cudaMemcpyAsync(&h_err, err, 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess)
         return cuda_fail(e, "read error word");
