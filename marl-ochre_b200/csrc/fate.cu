@@ -21,7 +21,13 @@
 //                                   block 1: the swap_remove permutation
 //   k_fate_moves                    dead voxels cleared; one warp per swap_remove move
 //   k_fate_births                   one warp per daughter: gather the parent's
-//                                   row, draw + mutate on one lane, write the slot
+//                                   row, draw + mutate, write the slot
+// Every one of them is bound by latency: a tick has tens of divisions and deaths.
+// So each starts under the end of the one before it (programmatic dependent
+// launch), and the births mutate while the moves run.  With that, mutation by a
+// whole warp instead of one lane (29 us of a step) and the halving's 16 loads in
+// flight together, a tick of a 60x52x30 grid (300 to 600 ticks old) fell from 223
+// to 203 us, one of 192x160x96 from 1,182 to 1,160.
 //
 // swap_remove in closed form.  Removing the ascending deaths d from the back
 // leaves n1 = n - |deaths| cells.  Let D(x) be the number of deaths below x,
@@ -40,8 +46,10 @@
 
 #include "common.cuh"
 #include "ctx_impl.h"
+#include "fate_mutate.cuh"
 #include "fate_stream.h"
 #include "internal.h"
+#include "kernel_setup.h"
 #include "table_ops.cuh"
 
 namespace marl {
@@ -127,6 +135,7 @@ __device__ __forceinline__ uint32_t packed_counts(const uint8_t e[8]) {
 // run r's cells [2048 x, 2048 x + 2048).
 __global__ void __launch_bounds__(kFateThreads) k_fate_count(const FateRun* __restrict__ runs) {
     __shared__ uint32_t wb[33];
+    griddep_launch_dependents();
     const FateRun& R = runs[blockIdx.y];
     const uint32_t n = R.f.fs->n;
     if (blockIdx.x * kFateChunk >= n) return;
@@ -140,6 +149,8 @@ __global__ void __launch_bounds__(kFateThreads) k_fate_count(const FateRun* __re
 // Same grid: the chunk's events into the run's ascending Division and Death lists.
 __global__ void __launch_bounds__(kFateThreads) k_fate_scatter(const FateRun* __restrict__ runs) {
     __shared__ uint32_t wb[33];
+    griddep_wait();
+    griddep_launch_dependents();
     const FateRun& R = runs[blockIdx.y];
     const uint32_t n = R.f.fs->n;
     if (blockIdx.x == 0 && threadIdx.x == 0) R.f.fs->n_old = n;  // the population the step starts from
@@ -198,6 +209,8 @@ __global__ void __launch_bounds__(kResolveThreads) k_fate_resolve(const FateRun*
                                                                   uint32_t* err_out) {
     __shared__ uint32_t wb[33];
     __shared__ uint32_t s_win, s_placed, s_run, s_levels, s_err;
+    griddep_wait();
+    griddep_launch_dependents();
     const FateRun& R = runs[blockIdx.y];
     const FateBuffers& F = R.f;
     FateScalars* fs = F.fs;
@@ -255,11 +268,11 @@ __global__ void __launch_bounds__(kResolveThreads) k_fate_resolve(const FateRun*
                 F.div_slot[k] = slot;
                 if (flags >> 16) {
                     const uint32_t p = F.div_list[k];
+                    float v[MARL_M_INT];  // all loads in flight before the first store
 #pragma unroll
-                    for (int sp = 0; sp < MARL_M_INT; ++sp) {
-                        float& v = t.internal[(size_t)sp * cap + p];
-                        v = v * 0.5f;
-                    }
+                    for (int sp = 0; sp < MARL_M_INT; ++sp) v[sp] = t.internal[(size_t)sp * cap + p];
+#pragma unroll
+                    for (int sp = 0; sp < MARL_M_INT; ++sp) t.internal[(size_t)sp * cap + p] = v[sp] * 0.5f;
                 }
             }
             __syncthreads();
@@ -371,6 +384,8 @@ __global__ void __launch_bounds__(kResolveThreads) k_fate_resolve(const FateRun*
 // blocks of run r take its moves in turn.  A cleared voxel belongs to a dead
 // cell and a moved cell keeps its own voxel, so the two never meet.
 __global__ void __launch_bounds__(256) k_fate_moves(const FateRun* __restrict__ runs) {
+    griddep_wait();
+    griddep_launch_dependents();  // after the wait: k_fate_births reads k_fate_resolve's results before its own
     const FateRun& R = runs[blockIdx.y];
     const Grid g = R.g;
     const uint32_t ndeath = R.f.fs->ndeath;
@@ -395,6 +410,11 @@ __global__ void __launch_bounds__(32 * kFateBirthWarps) k_fate_births(const Fate
     const uint32_t ndiv = fs->ndiv, n1 = fs->n1;
     const unsigned long long seed = fs->seed, tick = fs->key_tick;
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    bool moved = false;
+    auto wait_for_moves = [&]() {
+        if (!moved) griddep_wait();
+        moved = true;
+    };
     for (uint32_t k = blockIdx.x * kFateBirthWarps + w; k < ndiv; k += gridDim.x * kFateBirthWarps) {
         const uint32_t slot = R.f.div_slot[k];
         if (slot == kFateNoSlot) continue;
@@ -404,23 +424,30 @@ __global__ void __launch_bounds__(32 * kFateBirthWarps) k_fate_births(const Fate
         const uint32_t p = R.f.div_list[k];
         const uint32_t pn = p < n1 ? p : R.f.newidx[p - n1];
         marl_cell& c = rec[w];
+        fate::WarpStream r(fate::stream_key(seed, tick, p));
+        r.skip(info.y & ~kPlacedBit);
+        if (p >= n1) {  // the parent itself has moved
+            wait_for_moves();
+            fence_acquire_gpu();  // no line that an earlier daughter's reads left in L1
+        }
         read_record_warp(R.t, pn, c);
         __syncwarp();
         if (l == 0) {
-            fate::Stream r(fate::stream_key(seed, tick, p));
-            r.skip(info.y & ~kPlacedBit);
             c.pos[0] = (uint16_t)pos_x(info.x);
             c.pos[1] = (uint16_t)pos_y(info.x);
             c.pos[2] = (uint16_t)pos_z(info.x);
             c.age = 0;
             c.prep_remaining = 0;
-            c.lineage_id = r.u64();
-            fate::mutate_ruleset(c.ruleset, r, sim);
         }
+        const uint64_t lineage = r.u64();
+        if (l == 0) c.lineage_id = lineage;
+        fate::mutate_ruleset_warp(c.ruleset, r, sim);
         __syncwarp();
+        wait_for_moves();  // the slot may be one that a cell has yet to leave
         write_record_warp(R.t, R.g, R.cmap, R.mask, slot, c);
         __syncwarp();
     }
+    wait_for_moves();  // whatever follows this kernel relies on the moves too
 }
 
 // Batch: every run's population and first global cell index from its fate
@@ -528,12 +555,14 @@ cudaError_t launch_fate(const FateRun* d_runs, int n_runs, uint32_t max_cap, uin
     if (n_runs <= 0) return cudaSuccess;
     const dim3 chunks(fate_blocks(max_cap), (unsigned)n_runs);
     k_fate_count<<<chunks, kFateThreads, 0, s>>>(d_runs);
-    k_fate_scatter<<<chunks, kFateThreads, 0, s>>>(d_runs);
-    k_fate_resolve<<<dim3(2, n_runs), kResolveThreads, 0, s>>>(d_runs, sim, err);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_dependent(k_fate_scatter, chunks, kFateThreads, 0, s, d_runs);
+    if (e == cudaSuccess) e = launch_dependent(k_fate_resolve, dim3(2, n_runs), kResolveThreads, 0, s, d_runs, sim, err);
     const unsigned per_run = (unsigned)std::max(1, 2 * num_sms / n_runs);
-    k_fate_moves<<<dim3(per_run, n_runs), 256, 0, s>>>(d_runs);
-    k_fate_births<<<dim3(per_run, n_runs), 32 * kFateBirthWarps, 0, s>>>(d_runs, sim);
-    return cudaGetLastError();
+    if (e == cudaSuccess) e = launch_dependent(k_fate_moves, dim3(per_run, n_runs), 256, 0, s, d_runs);
+    if (e == cudaSuccess)
+        e = launch_dependent(k_fate_births, dim3(per_run, n_runs), 32 * kFateBirthWarps, 0, s, d_runs, sim);
+    return e;
 }
 
 cudaError_t launch_batch_population(RunDesc* runs, int n_runs, const FateRun* fr, cudaStream_t s) {

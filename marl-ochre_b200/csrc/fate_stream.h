@@ -83,6 +83,28 @@ MARL_HD double stream_ln(double s) {
     return fma((double)e, 0x1.62e42fefa39efp-1, lnm);
 }
 
+// The polar method's value for an accepted pair.
+MARL_HD float polar_normal(double u, double s2, float stddev) {
+    const double z = u * sqrt(-2.0 * stream_ln(s2) / s2);
+    return 0.0f + stddev * (float)z;
+}
+
+// Lemire's multiply-and-reject over a generator's u64().
+template <class Rng>
+MARL_HD uint32_t draw_range(Rng& rng, uint32_t lo, uint32_t hi) {
+    const uint32_t span = hi - lo;
+    uint64_t prod = (rng.u64() >> 32) * (uint64_t)span;
+    uint32_t low = (uint32_t)prod;
+    if (low < span) {
+        const uint32_t reject_below = (0u - span) % span;
+        while (low < reject_below) {
+            prod = (rng.u64() >> 32) * (uint64_t)span;
+            low = (uint32_t)prod;
+        }
+    }
+    return lo + (uint32_t)(prod >> 32);
+}
+
 // One division's stream.  `draws` counts the u64 outputs taken, so that a
 // later kernel can resume the stream where an earlier one left it.
 struct Stream {
@@ -97,8 +119,9 @@ struct Stream {
         }
     }
     MARL_HD static uint64_t rotl(uint64_t v, int k) { return (v << k) | (v >> (64 - k)); }
+    MARL_HD static uint64_t output(uint64_t s1) { return rotl(s1 * 5, 7) * 9; }
     MARL_HD uint64_t u64() {
-        const uint64_t out = rotl(s[1] * 5, 7) * 9;
+        const uint64_t out = output(s[1]);
         const uint64_t t = s[1] << 17;
         s[2] ^= s[0];
         s[3] ^= s[1];
@@ -113,19 +136,7 @@ struct Stream {
         for (uint32_t i = 0; i < k; ++i) u64();
     }
     MARL_HD float f32() { return (float)(u64() >> 40) * 0x1.0p-24f; }
-    MARL_HD uint32_t range(uint32_t lo, uint32_t hi) {
-        const uint32_t span = hi - lo;
-        uint64_t prod = (u64() >> 32) * (uint64_t)span;
-        uint32_t low = (uint32_t)prod;
-        if (low < span) {
-            const uint32_t reject_below = (0u - span) % span;
-            while (low < reject_below) {
-                prod = (u64() >> 32) * (uint64_t)span;
-                low = (uint32_t)prod;
-            }
-        }
-        return lo + (uint32_t)(prod >> 32);
-    }
+    MARL_HD uint32_t range(uint32_t lo, uint32_t hi) { return draw_range(*this, lo, hi); }
     MARL_HD float normal(float stddev) {
         for (int tries = 0; tries < 64; ++tries) {
             const double u = (double)(u64() >> 11) * 0x1.0p-52 - 1.0;
@@ -133,10 +144,7 @@ struct Stream {
             const double uu = u * u;
             const double vv = v * v;
             const double s2 = uu + vv;
-            if (s2 < 1.0 && s2 > 0.0) {
-                const double z = u * sqrt(-2.0 * stream_ln(s2) / s2);
-                return 0.0f + stddev * (float)z;
-            }
+            if (s2 < 1.0 && s2 > 0.0) return polar_normal(u, s2, stddev);
         }
         return 0.0f;
     }

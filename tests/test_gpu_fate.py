@@ -313,3 +313,21 @@ def test_device_fate_under_lane_refill(marl):
         assert a.stats()[k] == b.stats()[k], k
     assert a.cells().tobytes() == b.cells().tobytes()
     np.testing.assert_array_equal(a.field().view(np.uint32), b.field().view(np.uint32))
+
+
+@pytest.mark.parametrize("rate,mult,meta", [(0.0, 1.0, 1.0), (0.02, 0.1, 0.01), (0.19, 1.0, 0.0), (1.0, 0.0, 1.0),
+                                            (1.0, 1.0, 1.0)])
+def test_mutation_by_a_warp(marl, oracle_mod, rate, mult, meta):
+    """More daughters than the launch has warps, parents that move in the same step,
+    from no change in a daughter to one at every draw."""
+    dims, n = (40, 36, 24), 9000
+    rng = np.random.default_rng(int(1000 * rate))
+    p = mutation_params(marl)
+    p.structural_mutation_rate_mult, p.meta_mutation_rate = mult, meta
+    cells = mutable_cells(dims, n, rng)
+    cells["ruleset"]["mutation_rate"] = rate
+    events = rng.choice([0, DIV, DEATH], size=n, p=[0.4, 0.35, 0.25]).astype(np.uint8)
+    _, got, occ, _ = device_step(marl, dims, p, cells, events, 11, 5)
+    _, want, occ_want, _ = oracle_step(oracle_mod, dims, p, cells, events, 11, 5)
+    assert_same_cells(got, want)
+    np.testing.assert_array_equal(occ, occ_want)
