@@ -82,7 +82,7 @@ struct TrainArgs {
     const __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr;
     const float* p = nullptr;          // FP32 parameters (the biases are read)
     __nv_bfloat16 *h1 = nullptr, *h2 = nullptr, *dy = nullptr, *dz2 = nullptr, *dz1 = nullptr;
-    float *d1 = nullptr, *d2 = nullptr;  // GELU' of the pre-activations [B][256]
+    float* d1 = nullptr;               // GELU' of layer 1's pre-activations [B][256]
     float* y = nullptr;                // [B][16]
     uint32_t split_rows = 0;           // rows of a weight-gradient partial sum (train_split_rows)
     float* weight_part = nullptr;      // [splits][kParams]: the weights' partial sums

@@ -1,6 +1,6 @@
-// Training step of the reaction surrogate on the fifth-generation tensor cores:
-// six kernels (forward 1, forward 2, output layer with the loss, two input
-// gradients, all weight gradients) and Adam.
+// Training step of the reaction surrogate on the fifth-generation tensor cores, in
+// three kernels: everything that goes row by row (three layers, loss, input
+// gradients), all weight gradients, and Adam.
 //
 //   h1 = gelu(x W1^T + b1)      rows of x drawn from the prepared pairs
 //   h2 = gelu(h1 W2^T + b2)
@@ -15,18 +15,18 @@
 // zeroed or accumulated into by atomics.
 //
 // What bounds a step is latency: 4.6 GFLOP at a batch of 8192 are 3 us of the
-// tensor cores.  So each kernel spreads over as many SMs as the shape gives
-// (128 x 128 tiles: 128 blocks a layer, 8 x 16 blocks for the weight
-// gradients), has all its operand chunks in flight at once, and starts under
-// the tail of the one before it (programmatic dependent launch).  No operand is
-// transposed in memory: where a matrix is contracted over its rows, the tensor
-// core reads it as it lies (operands contiguous in M or N, the descriptor's
-// MN-major form).  The forward epilogues store gelu' from the tanh they have
-// already taken, so the backward ones take none.  The batch is never copied:
-// its rows are drawn by the loads that use them.
-// A step at a batch of 8192 takes 62 us (46 at 1024); it took 347 (295) as 14
-// kernels with transposed copies, shared-memory atomics in the loss (75 us) and
-// 60-us input-gradient epilogues.
+// tensor cores.  So each kernel spreads over as many SMs as the shape gives (128
+// blocks at 8192 for the rows, 8 x 16 for the weight gradients), has its operand
+// chunks in flight at once, and starts under the tail of the one before it
+// (programmatic dependent launch).  No operand is transposed in memory: where a
+// matrix is contracted over its rows, the tensor core reads it as it lies
+// (operands contiguous in M or N, the descriptor's MN-major form).  The forward
+// epilogues take gelu' from the tanh they have already taken, so the backward
+// ones take none.  The batch is never copied: its rows are drawn by the loads that
+// use them.
+// A step takes 53 us at a batch of 8192 (50 at 512, 336 at 65,536).  With a kernel
+// per layer and direction it took 71 (55, 372); as 14 kernels with transposed
+// copies and shared-memory atomics in the loss, 347 at 8192.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -51,10 +51,10 @@ __device__ __forceinline__ void cp_async_wait() {
 __device__ __forceinline__ void cp_async_commit_group() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 
 // Chunk of 64 k of `rows` rows (row r at src + at(r) * ld), K-major.
-template <class At>
+template <int THREADS, class At>
 __device__ __forceinline__ void stage_k(uint32_t dst, const __nv_bfloat16* src, int ld, int rows, int k0, int pieces,
                                         At at) {
-    for (int p = threadIdx.x; p < rows * pieces; p += kTrThreads) {
+    for (int p = threadIdx.x; p < rows * pieces; p += THREADS) {
         const int r = p / pieces, q = p % pieces;
         cp_async16_zfill(dst + r * 128 + ((q ^ (r & 7)) << 4), src + (size_t)at(r) * ld + k0 + q * 8, 16u);
     }
@@ -62,10 +62,10 @@ __device__ __forceinline__ void stage_k(uint32_t dst, const __nv_bfloat16* src, 
 
 // Rows at(0..krows-1) of a row-major matrix as k, columns n0 .. n0 + 8 pieces - 1
 // as the operand's M or N: MN-major, blocks of 64 columns.
-template <class At>
+template <int THREADS, class At>
 __device__ __forceinline__ void stage_mn(uint32_t dst, const __nv_bfloat16* src, int ld, int krows, int n0, int pieces,
                                          At at) {
-    for (int p = threadIdx.x; p < krows * pieces; p += kTrThreads) {
+    for (int p = threadIdx.x; p < krows * pieces; p += THREADS) {
         const int r = p / pieces, q = p % pieces;
         cp_async16_zfill(dst + (q >> 3) * kMnBlock + r * 128 + (((q & 7) ^ (r & 7)) << 4),
                          src + (size_t)at(r) * ld + n0 + q * 8, 16u);
@@ -76,11 +76,12 @@ struct TrSetup {
     uint32_t tmem, base;
 };
 
-// Tensor memory (kTrN columns), `bars` barriers, 1024-byte aligned staging.
+// Tensor memory (COLS columns), `bars` barriers, 1024-byte aligned staging.
+template <uint32_t COLS>
 __device__ __forceinline__ TrSetup tr_setup(uint8_t* raw, uint64_t* bars, int n_bars, uint32_t* slot) {
     if (threadIdx.x < 32) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(slot)),
-                     "r"((uint32_t)kTrN)
+                     "r"(COLS)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
@@ -94,11 +95,12 @@ __device__ __forceinline__ TrSetup tr_setup(uint8_t* raw, uint64_t* bars, int n_
     return TrSetup{*slot, (smem_u32(raw) + 1023u) & ~1023u};
 }
 
+template <uint32_t COLS>
 __device__ __forceinline__ void tr_teardown(uint32_t tmem) {
     tc_fence_before();
     __syncthreads();
     if (threadIdx.x < 32)
-        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)kTrN)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(COLS)
                      : "memory");
 }
 
@@ -130,172 +132,272 @@ __device__ __forceinline__ uint32_t drawn_row(const TrainArgs& a, uint32_t r) {
     return a.n_rows ? (uint32_t)(mix64(a.seed ^ mix64(a.step * 0x100000001B3ull + r)) % a.n_rows) : r;
 }
 
-enum TrRows : int { TR_FORWARD1, TR_FORWARD2, TR_LOSS, TR_BACK2, TR_BACK1 };
+// Everything of a step that goes row by row: three layers forward, the loss, two
+// backward.  A cluster of two blocks owns 128 rows; each block computes 128 of a
+// layer's 256 columns, so that 8192 rows are 128 blocks, and writes what the next
+// layer reads (H1, then H2, then dZ2) into both blocks' shared memory.  The
+// weights it needs are all staged at the start.  gelu' of layer 2 stays in tensor
+// memory; layer 1's goes to memory and comes back to the thread that wrote it.
+//
+// 16 warps: warp w reads tensor-memory lanes 32 (w % 4).. (tile rows) and columns
+// 32 (w / 4).. of its block's 128.
+constexpr int kRowThreads = 512;
+constexpr uint32_t kRowTmem = 256;              // columns 0-127 and 128-255: an accumulator each
+constexpr uint32_t kRowW2F = 0;                 // W2's own rows, K-major (forward), four chunks of 64 k
+constexpr uint32_t kRowW2B = 4 * kTile;         // W2's own columns, MN-major (backward), likewise
+constexpr uint32_t kRowH = 8 * kTile;           // X and W1, then H1, H2, dZ2: four chunks of 64 k
+constexpr uint32_t kRowW3 = 12 * kTile;         // four chunks [16][64]: K-major forward, MN-major backward
+constexpr uint32_t kRowW3Chunk = kOut * 128;
+constexpr uint32_t kRowDy = kRowW3 + 4 * kRowW3Chunk;
+constexpr uint32_t kRowSmem = kRowDy + kTile + 1024;
 
-// One layer over the batch's rows: a block owns 128 rows and N columns, with all
-// K (16, 128 or 256) staged at once, a commit group per chunk.  Eight warps:
-// warp w reads tensor-memory lanes 32 (w % 4).. (tile rows) and the column half
-// w / 4.
-template <int KIND>
-__global__ void __launch_bounds__(kTrThreads) k_train_rows(const __grid_constant__ TrainArgs a) {
-    constexpr bool kFwd = KIND == TR_FORWARD1 || KIND == TR_FORWARD2;
-    constexpr bool kBack = KIND == TR_BACK1 || KIND == TR_BACK2;
-    constexpr int N = KIND == TR_LOSS ? kOut : kTrN;
-    constexpr int K = KIND == TR_FORWARD1 ? kInPad : (KIND == TR_BACK2 ? kOut : kHid);
-    constexpr int kChunks = K < kBK ? 1 : K / kBK;
-    constexpr int kSteps = (K < kBK ? K : kBK) / 16;  // MMAs a chunk
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+__device__ __forceinline__ uint32_t cluster_map(uint32_t saddr, uint32_t rank) {
+    uint32_t r;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(saddr), "r"(rank));
+    return r;
+}
+__device__ __forceinline__ void cluster_store(uint32_t addr, uint4 v) {
+    asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+                 : "memory");
+}
+// Generic writes (either block's shared memory) before asynchronous reads.
+__device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
+    k_train_rows(const __grid_constant__ TrainArgs a) {
     extern __shared__ uint8_t raw[];
     __shared__ uint64_t bar;
     __shared__ uint32_t slot;
     __shared__ uint32_t s_idx[kBM];
-    __shared__ float s_col[4][kTrN], s_bias[kTrN], s_loss[4];
+    __shared__ float s_col[2][4][kTrN], s_col3[4][kOut], s_b1[kTrN], s_b2[kTrN], s_b3[kOut], s_loss[4];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int m0 = blockIdx.x * kBM, n0 = blockIdx.y * N;
-    const TrSetup t = tr_setup(raw, &bar, 1, &slot);
-    constexpr uint32_t kStage = 2 * kTile;
-    auto sa = [&](int c) { return t.base + c * kStage; };
-    auto sb = [&](int c) { return t.base + c * kStage + kTile; };
+    const uint32_t rank = blockIdx.x & 1u;
+    const int m0 = (int)(blockIdx.x >> 1) * kBM, n0 = (int)rank * kTrN;
+    const TrSetup t = tr_setup<kRowTmem>(raw, &bar, 1, &slot);
+    const uint32_t w2f = t.base + kRowW2F, w2b = t.base + kRowW2B, H = t.base + kRowH, w3 = t.base + kRowW3,
+                   dy = t.base + kRowDy, peer = cluster_map(H, rank ^ 1u);
+    if (tid < kBM) s_idx[tid] = drawn_row(a, (uint32_t)(m0 + tid));
+    griddep_wait();  // Adam's weights
+    griddep_launch_dependents();
+    if (tid < kBM && rank == 0) a.idx[m0 + tid] = s_idx[tid];
+    if (tid < kTrN) s_b1[tid] = a.p[kOffB1 + n0 + tid], s_b2[tid] = a.p[kOffB2 + n0 + tid];
+    if (tid < kOut) s_b3[tid] = a.p[kOffB3 + tid];
+    __syncthreads();
     auto self = [](int r) { return r; };
-
-    // Weights and biases were written by Adam before the kernel in front of
-    // this one began (each waits for its predecessor before it lets the next
-    // start), so they are staged ahead of the wait; forward 1 follows Adam
-    // itself.
-    auto stage_b = [&](int c) {
-        if constexpr (KIND == TR_FORWARD1)
-            stage_k(sb(c), a.w1 + (size_t)n0 * kInPad, kInPad, N, c * kBK, 8, self);
-        else if constexpr (KIND == TR_FORWARD2)
-            stage_k(sb(c), a.w2 + (size_t)n0 * kHid, kHid, N, c * kBK, 8, self);
-        else if constexpr (KIND == TR_LOSS)
-            stage_k(sb(c), a.w3, kHid, N, c * kBK, 8, self);
-        else if constexpr (KIND == TR_BACK2)
-            stage_mn(sb(c), a.w3, kHid, kOut, n0, 16, self);
-        else
-            stage_mn(sb(c), a.w2 + (size_t)c * kBK * kHid, kHid, kBK, n0, 16, self);
-    };
-    auto stage_a = [&](int c) {
-        if constexpr (KIND == TR_FORWARD1)
-            stage_k(sa(c), a.X, kInPad, kBM, c * kBK, 8, [&](int r) { return s_idx[r]; });
-        else if constexpr (KIND == TR_BACK2)
-            stage_k(sa(c), a.dy + (size_t)m0 * kOut, kOut, kBM, 0, 2, self);
-        else
-            stage_k(sa(c), (KIND == TR_FORWARD2 ? a.h1 : (KIND == TR_LOSS ? a.h2 : a.dz2)) + (size_t)m0 * kHid, kHid,
-                    kBM, c * kBK, 8, self);
-    };
-    const float* bias = a.p + (KIND == TR_FORWARD1 ? kOffB1 : (KIND == TR_FORWARD2 ? kOffB2 : kOffB3));
-    if constexpr (KIND == TR_FORWARD1) {
-        if (tid < kBM) s_idx[tid] = drawn_row(a, (uint32_t)(m0 + tid));
-        griddep_wait();
-        griddep_launch_dependents();
-        if (tid < kBM && blockIdx.y == 0) a.idx[m0 + tid] = s_idx[tid];
-        __syncthreads();
-    } else {
 #pragma unroll
-        for (int c = 0; c < kChunks; ++c) stage_b(c);
-        griddep_wait();
-        griddep_launch_dependents();
-    }
-    if constexpr (!kBack)
-        if (tid < N) s_bias[tid] = bias[n0 + tid];
-    float* const part = a.row_part + (size_t)blockIdx.x * kTrRowSums;
-#pragma unroll
-    for (int c = 0; c < kChunks; ++c) {
-        if constexpr (KIND == TR_FORWARD1) stage_b(c);
-        stage_a(c);
+    for (int c = 0; c < 2; ++c) {
+        stage_k<kRowThreads>(H + c * kTile, a.X, kInPad, kBM, c * kBK, 8, [&](int r) { return s_idx[r]; });
+        stage_k<kRowThreads>(H + (2 + c) * kTile, a.w1 + (size_t)n0 * kInPad, kInPad, kTrN, c * kBK, 8, self);
         cp_async_commit_group();
     }
-    constexpr uint32_t idesc = idesc_bf16(kBM, N) | (kBack ? kIdescBMn : 0u);
 #pragma unroll
-    for (int c = 0; c < kChunks; ++c) {
-        if (c == 0) cp_async_wait<kChunks - 1>();
-        if (c == 1) cp_async_wait<(kChunks > 2 ? kChunks - 2 : 0)>();
-        if (c == 2) cp_async_wait<(kChunks > 3 ? kChunks - 3 : 0)>();
-        if (c == 3) cp_async_wait<0>();
+    for (int c = 0; c < 4; ++c)
+        stage_k<kRowThreads>(w2f + c * kTile, a.w2 + (size_t)n0 * kHid, kHid, kTrN, c * kBK, 8, self);
+    cp_async_commit_group();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+        stage_k<kRowThreads>(w3 + c * kRowW3Chunk, a.w3, kHid, kOut, c * kBK, 8, self);
+        stage_mn<kRowThreads>(w2b + c * kTile, a.w2 + (size_t)c * kBK * kHid, kHid, kBK, n0, 16, self);
+    }
+    cp_async_commit_group();
+
+    const uint32_t d0 = t.tmem, d1 = t.tmem + kTrN;  // the accumulators
+    const uint32_t idesc = idesc_bf16(kBM, kTrN), idesc_back = idesc | kIdescBMn;
+    // Layer 1: X (128 k) by W1's own rows.
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        if (c == 0) cp_async_wait<3>();
+        else cp_async_wait<2>();
         fence_proxy_async_smem();
         __syncthreads();
         if (tid == 0) {
             tc_fence_after();
 #pragma unroll
-            for (int kk = 0; kk < kSteps; ++kk)
-                umma_bf16(t.tmem, sw128_desc(sa(c) + kk * 32),
-                          kBack ? sw128_desc_mn(sb(c) + kk * 2048, kMnBlock) : sw128_desc(sb(c) + kk * 32), idesc,
+            for (int kk = 0; kk < 4; ++kk)
+                umma_bf16(d0, sw128_desc(H + c * kTile + kk * 32), sw128_desc(H + (2 + c) * kTile + kk * 32), idesc,
                           (c > 0 || kk > 0) ? 1u : 0u);
-            if (c == kChunks - 1) umma_commit(&bar);
+            if (c == 1) umma_commit(&bar);
         }
     }
-    const bool ok = wait_commit(&bar, 0, a.err);
+    bool ok = wait_commit(&bar, 0, a.err);
     tc_fence_after();
+    cluster_arrive();
+    cluster_wait();  // neither block reads X or W1 any more: H1 may take their place
 
-    const int quarter = warp & 3, half = warp >> 2;
-    const int row = m0 + quarter * 32 + lane;
-    const uint32_t t_lane = t.tmem + ((uint32_t)(quarter * 32) << 16);
-    if constexpr (KIND == TR_LOSS) {
-        if (half == 0) {
-            float v[16], g[16];
-            tmem_ld16(t_lane, v);
-            const float4* tp = reinterpret_cast<const float4*>(a.T + (size_t)(a.n_rows ? a.idx[row] : row) * kOut);
-            float4* yp = reinterpret_cast<float4*>(a.y + (size_t)row * kOut);
-            const float sc = 2.0f / ((float)a.B * 16.0f);
-            float loss = 0.0f;
+    const int quarter = warp & 3, c_lo = (warp >> 2) * 32;
+    const int rl = quarter * 32 + lane, row = m0 + rl;
+    const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+    // 16 columns (from column `col` of 256) of this thread's row into both blocks' H.
+    auto put = [&](int col, const float (&h)[16]) {
+        const uint32_t at = (uint32_t)(col >> 6) * kTile + (uint32_t)rl * 128, q = (uint32_t)(col & 63) >> 3;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                const float4 tt = tp[q];
-                const float y0 = v[4 * q] + s_bias[4 * q], y1 = v[4 * q + 1] + s_bias[4 * q + 1],
-                            y2 = v[4 * q + 2] + s_bias[4 * q + 2], y3 = v[4 * q + 3] + s_bias[4 * q + 3];
-                const float e0 = y0 - tt.x, e1 = y1 - tt.y, e2 = y2 - tt.z, e3 = y3 - tt.w;
-                loss += e0 * e0 + e1 * e1 + e2 * e2 + e3 * e3;
-                g[4 * q] = ok ? e0 * sc : 0.0f, g[4 * q + 1] = ok ? e1 * sc : 0.0f;
-                g[4 * q + 2] = ok ? e2 * sc : 0.0f, g[4 * q + 3] = ok ? e3 * sc : 0.0f;
-                yp[q] = make_float4(y0, y1, y2, y3);
-            }
-            store_bf16x16(a.dy + (size_t)row * kOut, g);
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, o);
-            const float sum = column_sums16(g, lane);
-            if (!(lane & 1)) s_col[quarter][lane >> 1] = sum;
-            if (lane == 0) s_loss[quarter] = loss;
+        for (uint32_t i = 0; i < 2; ++i) {
+            const uint4 v = make_uint4(pack_bf16(h[8 * i], h[8 * i + 1]), pack_bf16(h[8 * i + 2], h[8 * i + 3]),
+                                       pack_bf16(h[8 * i + 4], h[8 * i + 5]), pack_bf16(h[8 * i + 6], h[8 * i + 7]));
+            const uint32_t to = at + (((q + i) ^ ((uint32_t)rl & 7u)) << 4);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(H + to), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+                         : "memory");
+            cluster_store(peer + to, v);
         }
-        __syncthreads();
-        if (tid < kOut) part[2 * kHid + tid] = (s_col[0][tid] + s_col[1][tid]) + (s_col[2][tid] + s_col[3][tid]);
-        if (tid == kOut) part[2 * kHid + kOut] = (s_loss[0] + s_loss[1]) + (s_loss[2] + s_loss[3]);
-    } else {
-        __nv_bfloat16* out = KIND == TR_FORWARD1 ? a.h1 : (KIND == TR_FORWARD2 ? a.h2 : (KIND == TR_BACK2 ? a.dz2 : a.dz1));
-        float* d = (KIND == TR_FORWARD1 || KIND == TR_BACK1) ? a.d1 : a.d2;
-#pragma unroll 1
-        for (int cb = half * (N / 2); cb < (half + 1) * (N / 2); cb += 16) {
-            float v[16], h[16];
-            const size_t at = (size_t)row * kHid + n0 + cb;
-            float4* dp = reinterpret_cast<float4*>(d + at);
-            if constexpr (kFwd) {
-                tmem_ld16(t_lane + cb, v);
+    };
+    // After it, both blocks have written H.
+    auto exchange = [&]() {
+        fence_proxy_async_all();
+        tc_fence_before();
+        cluster_arrive();
+        cluster_wait();
+    };
+    // D = H (256 k) by B's chunks.
+    auto mma_h = [&](uint32_t d, uint32_t idesc_n, auto bdesc) {
+        if (tid == 0) {
+            fence_proxy_async_all();
+            tc_fence_after();
 #pragma unroll
-                for (int i = 0; i < 16; ++i) h[i] = gelu_and_grad(v[i] + s_bias[cb + i], v[i]);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) dp[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-                store_bf16x16(out + at, h);
-            } else {
-                float4 dg[4];
-#pragma unroll
-                for (int q = 0; q < 4; ++q) dg[q] = dp[q];
-                tmem_ld16(t_lane + cb, v);
-#pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    h[4 * q] = ok ? v[4 * q] * dg[q].x : 0.0f, h[4 * q + 1] = ok ? v[4 * q + 1] * dg[q].y : 0.0f;
-                    h[4 * q + 2] = ok ? v[4 * q + 2] * dg[q].z : 0.0f, h[4 * q + 3] = ok ? v[4 * q + 3] * dg[q].w : 0.0f;
-                }
-                store_bf16x16(out + at, h);
-                const float sum = column_sums16(h, lane);
-                if (!(lane & 1)) s_col[quarter][cb + (lane >> 1)] = sum;
-            }
+            for (int k = 0; k < 16; ++k)
+                umma_bf16(d, sw128_desc(H + (k >> 2) * kTile + (k & 3) * 32), bdesc(k >> 2, k & 3), idesc_n, k > 0 ? 1u : 0u);
+            umma_commit(&bar);
         }
-        if constexpr (kBack) {
-            __syncthreads();
-            if (tid < N)
-                part[(KIND == TR_BACK2 ? kHid : 0) + n0 + tid] =
-                    (s_col[0][tid] + s_col[1][tid]) + (s_col[2][tid] + s_col[3][tid]);
-        }
+    };
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int cb = c_lo + 16 * i;
+        float v[16], h[16];
+        tmem_ld16(d0 + lanes + cb, v);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) h[j] = gelu_and_grad(v[j] + s_b1[cb + j], v[j]);
+        const size_t at = (size_t)row * kHid + n0 + cb;
+        float4* dp = reinterpret_cast<float4*>(a.d1 + at);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) dp[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+        store_bf16x16(a.h1 + at, h);
+        put(n0 + cb, h);
     }
-    tr_teardown(t.tmem);
+    cp_async_wait<1>();
+    exchange();
+    // Layer 2: H1 by W2's own rows.
+    mma_h(d1, idesc, [&](int c, int kk) { return sw128_desc(w2f + c * kTile + kk * 32); });
+    ok = wait_commit(&bar, 1, a.err) && ok;
+    tc_fence_after();
+    cluster_arrive();
+    cluster_wait();  // neither block reads H1 any more
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int cb = c_lo + 16 * i;
+        float v[16], h[16];
+        uint32_t g[16];
+        tmem_ld16(d1 + lanes + cb, v);
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            float grad;
+            h[j] = gelu_and_grad(v[j] + s_b2[cb + j], grad);
+            g[j] = __float_as_uint(grad);
+        }
+        tmem_st16(d1 + lanes + cb, g);
+        store_bf16x16(a.h2 + (size_t)row * kHid + n0 + cb, h);
+        put(n0 + cb, h);
+    }
+    tmem_st_wait();
+    cp_async_wait<0>();
+    exchange();
+    // Layer 3 and the loss, in both blocks alike; the first one writes them.
+    mma_h(d0, idesc_bf16(kBM, kOut), [&](int c, int kk) { return sw128_desc(w3 + c * kRowW3Chunk + kk * 32); });
+    ok = wait_commit(&bar, 0, a.err) && ok;
+    tc_fence_after();
+    cluster_arrive();  // this block reads H2 no more; waited for before dZ2 takes its place
+    if (warp < 4) {
+        float v[16], g[16];
+        tmem_ld16(d0 + lanes, v);
+        const float4* tp = reinterpret_cast<const float4*>(a.T + (size_t)s_idx[rl] * kOut);
+        float4* yp = reinterpret_cast<float4*>(a.y + (size_t)row * kOut);
+        const float sc = 2.0f / ((float)a.B * 16.0f);
+        float loss = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float4 tt = tp[q];
+            const float y0 = v[4 * q] + s_b3[4 * q], y1 = v[4 * q + 1] + s_b3[4 * q + 1],
+                        y2 = v[4 * q + 2] + s_b3[4 * q + 2], y3 = v[4 * q + 3] + s_b3[4 * q + 3];
+            const float e0 = y0 - tt.x, e1 = y1 - tt.y, e2 = y2 - tt.z, e3 = y3 - tt.w;
+            loss += e0 * e0 + e1 * e1 + e2 * e2 + e3 * e3;
+            g[4 * q] = ok ? e0 * sc : 0.0f, g[4 * q + 1] = ok ? e1 * sc : 0.0f;
+            g[4 * q + 2] = ok ? e2 * sc : 0.0f, g[4 * q + 3] = ok ? e3 * sc : 0.0f;
+            if (rank == 0) yp[q] = make_float4(y0, y1, y2, y3);
+        }
+        if (rank == 0) store_bf16x16(a.dy + (size_t)row * kOut, g);
+#pragma unroll
+        for (uint32_t i = 0; i < 2; ++i)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dy + (uint32_t)rl * 128 +
+                                                                          ((i ^ ((uint32_t)rl & 7u)) << 4)),
+                         "r"(pack_bf16(g[8 * i], g[8 * i + 1])), "r"(pack_bf16(g[8 * i + 2], g[8 * i + 3])),
+                         "r"(pack_bf16(g[8 * i + 4], g[8 * i + 5])), "r"(pack_bf16(g[8 * i + 6], g[8 * i + 7]))
+                         : "memory");
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) loss += __shfl_xor_sync(0xFFFFFFFFu, loss, o);
+        const float sum = column_sums16(g, lane);
+        if (!(lane & 1)) s_col3[quarter][lane >> 1] = sum;
+        if (lane == 0) s_loss[quarter] = loss;
+    }
+    fence_proxy_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    float* const part = a.row_part + (size_t)(blockIdx.x >> 1) * kTrRowSums;
+    // dH2's own columns: dY (16 k) by W3.
+    if (tid == 0) {
+        tc_fence_after();
+        umma_bf16(d0, sw128_desc(dy), sw128_desc_mn(w3 + 2 * rank * kRowW3Chunk, kRowW3Chunk), idesc_back, 0u);
+        umma_commit(&bar);
+    }
+    if (rank == 0 && tid < kOut)
+        part[2 * kHid + tid] = (s_col3[0][tid] + s_col3[1][tid]) + (s_col3[2][tid] + s_col3[3][tid]);
+    if (rank == 0 && tid == kOut) part[2 * kHid + kOut] = (s_loss[0] + s_loss[1]) + (s_loss[2] + s_loss[3]);
+    ok = wait_commit(&bar, 1, a.err) && ok;
+    tc_fence_after();
+    cluster_wait();
+    auto back = [&](int cb, float (&v)[16], const float (&dg)[16], __nv_bfloat16* out, float (&h)[16]) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) h[j] = ok ? v[j] * dg[j] : 0.0f;
+        store_bf16x16(out + (size_t)row * kHid + n0 + cb, h);
+    };
+    auto sums = [&](int which, int cb, float (&h)[16]) {
+        const float sum = column_sums16(h, lane);
+        if (!(lane & 1)) s_col[which][quarter][cb + (lane >> 1)] = sum;
+    };
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int cb = c_lo + 16 * i;
+        float v[16], dg[16], h[16];
+        tmem_ld16(d1 + lanes + cb, dg);
+        tmem_ld16(d0 + lanes + cb, v);
+        back(cb, v, dg, a.dz2, h);
+        put(n0 + cb, h);
+        sums(0, cb, h);
+    }
+    exchange();
+    // dH1's own columns: dZ2 by W2's columns.
+    mma_h(d1, idesc_back, [&](int c, int kk) { return sw128_desc_mn(w2b + c * kTile + kk * 2048, kMnBlock); });
+    if (tid < kTrN)
+        part[kHid + n0 + tid] = (s_col[0][0][tid] + s_col[0][1][tid]) + (s_col[0][2][tid] + s_col[0][3][tid]);
+    float dg[2][16];
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            *reinterpret_cast<float4*>(&dg[i][4 * q]) =
+                reinterpret_cast<const float4*>(a.d1 + (size_t)row * kHid + n0 + c_lo + 16 * i)[q];
+    ok = wait_commit(&bar, 0, a.err) && ok;
+    tc_fence_after();
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int cb = c_lo + 16 * i;
+        float v[16], h[16];
+        tmem_ld16(d1 + lanes + cb, v);
+        back(cb, v, dg[i], a.dz1, h);
+        sums(1, cb, h);
+    }
+    __syncthreads();
+    if (tid < kTrN) part[n0 + tid] = (s_col[1][0][tid] + s_col[1][1][tid]) + (s_col[1][2][tid] + s_col[1][3][tid]);
+    tr_teardown<kRowTmem>(t.tmem);
 }
 
 // The weight gradients: block (job, split) sums split_rows rows of the batch
@@ -312,7 +414,7 @@ __global__ void __launch_bounds__(kTrThreads) k_train_weights(const __grid_const
     __shared__ uint32_t slot;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int job = blockIdx.x;
-    const TrSetup t = tr_setup(raw, bars, kTrStages, &slot);
+    const TrSetup t = tr_setup<kTrN>(raw, bars, kTrStages, &slot);
     griddep_wait();
     griddep_launch_dependents();
     const int per = (int)(a.split_rows / kBK), c0 = (int)blockIdx.y * per, c1 = min(c0 + per, (int)(a.B / kBK));
@@ -324,13 +426,13 @@ __global__ void __launch_bounds__(kTrThreads) k_train_weights(const __grid_const
         const uint32_t sa = t.base + (uint32_t)((c - c0) & (kTrStages - 1)) * 2 * kTile, sb = sa + kTile;
         const int r0 = c * kBK;
         auto rows = [&](int r) { return r0 + r; };
-        stage_mn(sa, A, kHid, kBK, 0, 16, rows);
+        stage_mn<kTrThreads>(sa, A, kHid, kBK, 0, 16, rows);
         if (last_layer)
-            stage_mn(sb, a.dy, kOut, kBK, 0, 2, rows);
+            stage_mn<kTrThreads>(sb, a.dy, kOut, kBK, 0, 2, rows);
         else if (first_layer)
-            stage_mn(sb, a.X, kInPad, kBK, 0, 16, [&](int r) { return a.n_rows ? a.idx[r0 + r] : (uint32_t)(r0 + r); });
+            stage_mn<kTrThreads>(sb, a.X, kInPad, kBK, 0, 16, [&](int r) { return a.n_rows ? a.idx[r0 + r] : (uint32_t)(r0 + r); });
         else
-            stage_mn(sb, a.h1, kHid, kBK, (job & 1) * kTrN, 16, rows);
+            stage_mn<kTrThreads>(sb, a.h1, kHid, kBK, (job & 1) * kTrN, 16, rows);
     };
     const uint32_t idesc = (last_layer ? idesc_bf16(kBM, kOut) : idesc_bf16(kBM, kTrN)) | kIdescAMn | kIdescBMn;
     bool ok = true;
@@ -390,28 +492,16 @@ __global__ void __launch_bounds__(kTrThreads) k_train_weights(const __grid_const
             }
         }
     }
-    tr_teardown(t.tmem);
+    tr_teardown<kTrN>(t.tmem);
 }
 static_assert(kOffW1 % 4 == 0 && kOffW2 % 4 == 0 && kParams % 4 == 0, "four-wide stores");
 
-template <int KIND>
-static cudaError_t launch_rows(const TrainArgs& a, cudaStream_t s) {
-    constexpr int chunks = KIND == TR_FORWARD1 ? kInPad / kBK : (KIND == TR_BACK2 ? 1 : kHid / kBK);
-    constexpr int smem = chunks * 2 * kTile + 1024;
-    static std::atomic<int> setup[kSetupDevices];
-    cudaError_t e = set_smem_once(setup, k_train_rows<KIND>, smem);
-    if (e != cudaSuccess) return e;
-    return launch_dependent(k_train_rows<KIND>, dim3(a.B / kBM, KIND == TR_LOSS ? 1 : kHid / kTrN), dim3(kTrThreads),
-                            smem, s, a);
-}
-
 cudaError_t launch_forward_backward(const TrainArgs& a, cudaStream_t s) {
     if (a.B == 0 || a.B % kBM) return cudaErrorInvalidValue;
-    cudaError_t e = launch_rows<TR_FORWARD1>(a, s);
-    if (e == cudaSuccess) e = launch_rows<TR_FORWARD2>(a, s);
-    if (e == cudaSuccess) e = launch_rows<TR_LOSS>(a, s);
-    if (e == cudaSuccess) e = launch_rows<TR_BACK2>(a, s);
-    if (e == cudaSuccess) e = launch_rows<TR_BACK1>(a, s);
+    static std::atomic<int> setup_rows[kSetupDevices];
+    cudaError_t e = set_smem_once(setup_rows, k_train_rows, kRowSmem);
+    if (e == cudaSuccess)
+        e = launch_dependent(k_train_rows, dim3(2 * (a.B / kBM)), dim3(kRowThreads), kRowSmem, s, a);
     if (e != cudaSuccess) return e;
     static std::atomic<int> setup[kSetupDevices];
     if ((e = set_smem_once(setup, k_train_weights, kTrSmem)) != cudaSuccess) return e;
