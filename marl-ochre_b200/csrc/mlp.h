@@ -78,11 +78,11 @@ struct TrainArgs {
     const float* T = nullptr;          // their targets [.][16]
     uint32_t n_rows = 0;               // batch row r is a hashed draw from [0, n_rows); 0: row r itself
     uint64_t seed = 0, step = 0;       // of the draws
-    uint32_t* idx = nullptr;           // [B] the drawn rows
     const __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr;
     const float* p = nullptr;          // FP32 parameters (the biases are read)
-    __nv_bfloat16 *h1 = nullptr, *h2 = nullptr, *dy = nullptr, *dz2 = nullptr, *dz1 = nullptr;
-    float* d1 = nullptr;               // GELU' of layer 1's pre-activations [B][256]
+    // Images of 128-row, 64-column shared-memory tiles (16 KB, BF16): two to a row
+    // tile of X, four of h1, h2, dz2 and dz1, one (16 columns used) of dy.
+    uint8_t *xt = nullptr, *h1 = nullptr, *h2 = nullptr, *dy = nullptr, *dz2 = nullptr, *dz1 = nullptr;
     float* y = nullptr;                // [B][16]
     uint32_t split_rows = 0;           // rows of a weight-gradient partial sum (train_split_rows)
     float* weight_part = nullptr;      // [splits][kParams]: the weights' partial sums

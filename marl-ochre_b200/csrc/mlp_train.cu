@@ -24,9 +24,10 @@
 // epilogues take gelu' from the tanh they have already taken, so the backward
 // ones take none.  The batch is never copied: its rows are drawn by the loads that
 // use them.
-// A step takes 53 us at a batch of 8192 (50 at 512, 336 at 65,536).  With a kernel
-// per layer and direction it took 71 (55, 372); as 14 kernels with transposed
-// copies and shared-memory atomics in the loss, 347 at 8192.
+// A step takes 37 us at a batch of 8192 (35 at 512, 221 at 65,536).  With rows
+// written and read 16 bytes a thread instead of tile images it took 54 (50, 335),
+// with a kernel per layer and direction 71 (55, 372), as 14 kernels with transposed
+// copies and shared-memory atomics in the loss 347 at 8192.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -41,6 +42,7 @@ namespace mlp {
 constexpr int kTrThreads = 256;
 constexpr int kTrN = 128;                  // columns of a block's tile
 constexpr uint32_t kTile = kBM * 128;      // a staged 128 x 64 (or 64 x 128) BF16 operand: 16 KB
+constexpr uint32_t kImage = kTile;         // a tile's image in memory
 constexpr uint32_t kMnBlock = kBK * 128;   // 64 k-rows of 64 elements: the stride between MN-major blocks
 constexpr int kTrStages = 4;
 
@@ -120,13 +122,6 @@ __device__ __forceinline__ float column_sums16(float (&v)[16], int lane) {
     return v[0] + __shfl_xor_sync(0xFFFFFFFFu, v[0], 1);
 }
 
-__device__ __forceinline__ void store_bf16x16(__nv_bfloat16* dst, const float (&h)[16]) {
-    uint4* o = reinterpret_cast<uint4*>(dst);
-    o[0] = make_uint4(pack_bf16(h[0], h[1]), pack_bf16(h[2], h[3]), pack_bf16(h[4], h[5]), pack_bf16(h[6], h[7]));
-    o[1] = make_uint4(pack_bf16(h[8], h[9]), pack_bf16(h[10], h[11]), pack_bf16(h[12], h[13]),
-                      pack_bf16(h[14], h[15]));
-}
-
 // Batch row r's prepared row.
 __device__ __forceinline__ uint32_t drawn_row(const TrainArgs& a, uint32_t r) {
     return a.n_rows ? (uint32_t)(mix64(a.seed ^ mix64(a.step * 0x100000001B3ull + r)) % a.n_rows) : r;
@@ -136,13 +131,17 @@ __device__ __forceinline__ uint32_t drawn_row(const TrainArgs& a, uint32_t r) {
 // backward.  A cluster of two blocks owns 128 rows; each block computes 128 of a
 // layer's 256 columns, so that 8192 rows are 128 blocks, and writes what the next
 // layer reads (H1, then H2, then dZ2) into both blocks' shared memory.  The
-// weights it needs are all staged at the start.  gelu' of layer 2 stays in tensor
-// memory; layer 1's goes to memory and comes back to the thread that wrote it.
+// weights it needs are all staged at the start, and gelu' of layers 1 and 2 stays
+// in tensor memory.  What the weight gradients need leaves as images of the
+// shared-memory tiles (128 rows of 64 columns, swizzled, 16 KB), one bulk copy
+// each: k_train_weights loads halves of them (64 rows) the same way, and they are
+// its operands as they are.  Stored row by row, 16 bytes a thread, they took 12
+// wavefronts of 32 rows a thread and 6k cycles of an epilogue.
 //
 // 16 warps: warp w reads tensor-memory lanes 32 (w % 4).. (tile rows) and columns
 // 32 (w / 4).. of its block's 128.
 constexpr int kRowThreads = 512;
-constexpr uint32_t kRowTmem = 256;              // columns 0-127 and 128-255: an accumulator each
+constexpr uint32_t kRowTmem = 512;              // columns 0-127 and 128-255: an accumulator each; 256-383: gelu' of layer 1
 constexpr uint32_t kRowW2F = 0;                 // W2's own rows, K-major (forward), four chunks of 64 k
 constexpr uint32_t kRowW2B = 4 * kTile;         // W2's own columns, MN-major (backward), likewise
 constexpr uint32_t kRowH = 8 * kTile;           // X and W1, then H1, H2, dZ2: four chunks of 64 k
@@ -162,6 +161,18 @@ __device__ __forceinline__ void cluster_store(uint32_t addr, uint4 v) {
     asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
                  : "memory");
 }
+// Asynchronous copies of whole tile images; sizes and addresses are multiples of 16.
+__device__ __forceinline__ void image_store(void* dst, uint32_t src, uint32_t bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void image_stores_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
+__device__ __forceinline__ void image_stores_done() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
+__device__ __forceinline__ void image_load(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                 : "memory");
+}
 // Generic writes (either block's shared memory) before asynchronous reads.
 __device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
@@ -174,14 +185,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
     __shared__ float s_col[2][4][kTrN], s_col3[4][kOut], s_b1[kTrN], s_b2[kTrN], s_b3[kOut], s_loss[4];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t rank = blockIdx.x & 1u;
-    const int m0 = (int)(blockIdx.x >> 1) * kBM, n0 = (int)rank * kTrN;
+    const uint32_t tile = blockIdx.x >> 1;
+    const int m0 = (int)tile * kBM, n0 = (int)rank * kTrN;
     const TrSetup t = tr_setup<kRowTmem>(raw, &bar, 1, &slot);
     const uint32_t w2f = t.base + kRowW2F, w2b = t.base + kRowW2B, H = t.base + kRowH, w3 = t.base + kRowW3,
                    dy = t.base + kRowDy, peer = cluster_map(H, rank ^ 1u);
     if (tid < kBM) s_idx[tid] = drawn_row(a, (uint32_t)(m0 + tid));
     griddep_wait();  // Adam's weights
     griddep_launch_dependents();
-    if (tid < kBM && rank == 0) a.idx[m0 + tid] = s_idx[tid];
     if (tid < kTrN) s_b1[tid] = a.p[kOffB1 + n0 + tid], s_b2[tid] = a.p[kOffB2 + n0 + tid];
     if (tid < kOut) s_b3[tid] = a.p[kOffB3 + tid];
     __syncthreads();
@@ -203,7 +214,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
     }
     cp_async_commit_group();
 
-    const uint32_t d0 = t.tmem, d1 = t.tmem + kTrN;  // the accumulators
+    const uint32_t d0 = t.tmem, d1 = t.tmem + kTrN, g1 = t.tmem + 2 * kTrN;  // the accumulators, gelu'
     const uint32_t idesc = idesc_bf16(kBM, kTrN), idesc_back = idesc | kIdescBMn;
     // Layer 1: X (128 k) by W1's own rows.
 #pragma unroll
@@ -219,28 +230,40 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
                 umma_bf16(d0, sw128_desc(H + c * kTile + kk * 32), sw128_desc(H + (2 + c) * kTile + kk * 32), idesc,
                           (c > 0 || kk > 0) ? 1u : 0u);
             if (c == 1) umma_commit(&bar);
+            if (c == (int)rank) image_store(a.xt + ((size_t)tile * 2 + c) * kImage, H + c * kTile, kTile);
         }
     }
     bool ok = wait_commit(&bar, 0, a.err);
     tc_fence_after();
+    if (tid == 0) image_stores_read();
     cluster_arrive();
     cluster_wait();  // neither block reads X or W1 any more: H1 may take their place
 
     const int quarter = warp & 3, c_lo = (warp >> 2) * 32;
-    const int rl = quarter * 32 + lane, row = m0 + rl;
+    const int rl = quarter * 32 + lane;
     const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
-    // 16 columns (from column `col` of 256) of this thread's row into both blocks' H.
-    auto put = [&](int col, const float (&h)[16]) {
+    // 16 columns (from column `col` of 256) of this thread's row into an image of
+    // four chunks, or into the peer's H.
+    auto pieces = [&](int col, const float (&h)[16], auto store) {
         const uint32_t at = (uint32_t)(col >> 6) * kTile + (uint32_t)rl * 128, q = (uint32_t)(col & 63) >> 3;
 #pragma unroll
-        for (uint32_t i = 0; i < 2; ++i) {
-            const uint4 v = make_uint4(pack_bf16(h[8 * i], h[8 * i + 1]), pack_bf16(h[8 * i + 2], h[8 * i + 3]),
-                                       pack_bf16(h[8 * i + 4], h[8 * i + 5]), pack_bf16(h[8 * i + 6], h[8 * i + 7]));
-            const uint32_t to = at + (((q + i) ^ ((uint32_t)rl & 7u)) << 4);
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(H + to), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+        for (uint32_t i = 0; i < 2; ++i)
+            store(at + (((q + i) ^ ((uint32_t)rl & 7u)) << 4),
+                  make_uint4(pack_bf16(h[8 * i], h[8 * i + 1]), pack_bf16(h[8 * i + 2], h[8 * i + 3]),
+                             pack_bf16(h[8 * i + 4], h[8 * i + 5]), pack_bf16(h[8 * i + 6], h[8 * i + 7])));
+    };
+    auto put = [&](uint32_t image, int col, const float (&h)[16]) {
+        pieces(col, h, [&](uint32_t at, uint4 v) {
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(image + at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
                          : "memory");
-            cluster_store(peer + to, v);
-        }
+        });
+    };
+    auto put_peer = [&](int col, const float (&h)[16]) {
+        pieces(col, h, [&](uint32_t at, uint4 v) { cluster_store(peer + at, v); });
+    };
+    // This block's half of an image in H (or at `from`) to memory.
+    auto store_half = [&](uint8_t* images, uint32_t from) {
+        if (tid == 0) image_store(images + ((size_t)tile * 4 + 2 * rank) * kImage, from + 2 * rank * kTile, 2 * kTile);
     };
     // After it, both blocks have written H.
     auto exchange = [&]() {
@@ -267,19 +290,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
         tmem_ld16(d0 + lanes + cb, v);
 #pragma unroll
         for (int j = 0; j < 16; ++j) h[j] = gelu_and_grad(v[j] + s_b1[cb + j], v[j]);
-        const size_t at = (size_t)row * kHid + n0 + cb;
-        float4* dp = reinterpret_cast<float4*>(a.d1 + at);
+        uint32_t g[16];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) dp[q] = make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-        store_bf16x16(a.h1 + at, h);
-        put(n0 + cb, h);
+        for (int j = 0; j < 16; ++j) g[j] = __float_as_uint(v[j]);
+        tmem_st16(g1 + lanes + cb, g);
+        put(H, n0 + cb, h);
+        put_peer(n0 + cb, h);
     }
+    tmem_st_wait();
     cp_async_wait<1>();
     exchange();
     // Layer 2: H1 by W2's own rows.
     mma_h(d1, idesc, [&](int c, int kk) { return sw128_desc(w2f + c * kTile + kk * 32); });
+    store_half(a.h1, H);
     ok = wait_commit(&bar, 1, a.err) && ok;
     tc_fence_after();
+    if (tid == 0) image_stores_read();
     cluster_arrive();
     cluster_wait();  // neither block reads H1 any more
 #pragma unroll
@@ -295,22 +321,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
             g[j] = __float_as_uint(grad);
         }
         tmem_st16(d1 + lanes + cb, g);
-        store_bf16x16(a.h2 + (size_t)row * kHid + n0 + cb, h);
-        put(n0 + cb, h);
+        put(H, n0 + cb, h);
+        put_peer(n0 + cb, h);
     }
     tmem_st_wait();
     cp_async_wait<0>();
     exchange();
     // Layer 3 and the loss, in both blocks alike; the first one writes them.
     mma_h(d0, idesc_bf16(kBM, kOut), [&](int c, int kk) { return sw128_desc(w3 + c * kRowW3Chunk + kk * 32); });
+    store_half(a.h2, H);
     ok = wait_commit(&bar, 0, a.err) && ok;
     tc_fence_after();
+    if (tid == 0) image_stores_read();
     cluster_arrive();  // this block reads H2 no more; waited for before dZ2 takes its place
     if (warp < 4) {
         float v[16], g[16];
         tmem_ld16(d0 + lanes, v);
         const float4* tp = reinterpret_cast<const float4*>(a.T + (size_t)s_idx[rl] * kOut);
-        float4* yp = reinterpret_cast<float4*>(a.y + (size_t)row * kOut);
+        float4* yp = reinterpret_cast<float4*>(a.y + (size_t)(m0 + rl) * kOut);
         const float sc = 2.0f / ((float)a.B * 16.0f);
         float loss = 0.0f;
 #pragma unroll
@@ -324,7 +352,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
             g[4 * q + 2] = ok ? e2 * sc : 0.0f, g[4 * q + 3] = ok ? e3 * sc : 0.0f;
             if (rank == 0) yp[q] = make_float4(y0, y1, y2, y3);
         }
-        if (rank == 0) store_bf16x16(a.dy + (size_t)row * kOut, g);
 #pragma unroll
         for (uint32_t i = 0; i < 2; ++i)
             asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dy + (uint32_t)rl * 128 +
@@ -347,6 +374,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
         tc_fence_after();
         umma_bf16(d0, sw128_desc(dy), sw128_desc_mn(w3 + 2 * rank * kRowW3Chunk, kRowW3Chunk), idesc_back, 0u);
         umma_commit(&bar);
+        if (rank == 0) image_store(a.dy + (size_t)tile * kImage, dy, kTile);
     }
     if (rank == 0 && tid < kOut)
         part[2 * kHid + tid] = (s_col3[0][tid] + s_col3[1][tid]) + (s_col3[2][tid] + s_col3[3][tid]);
@@ -354,10 +382,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
     ok = wait_commit(&bar, 1, a.err) && ok;
     tc_fence_after();
     cluster_wait();
-    auto back = [&](int cb, float (&v)[16], const float (&dg)[16], __nv_bfloat16* out, float (&h)[16]) {
+    // dZ = dH gelu'.
+    auto back = [&](uint32_t d, uint32_t g, int cb, float (&h)[16]) {
+        float v[16], dg[16];
+        tmem_ld16(g + lanes + cb, dg);
+        tmem_ld16(d + lanes + cb, v);
 #pragma unroll
         for (int j = 0; j < 16; ++j) h[j] = ok ? v[j] * dg[j] : 0.0f;
-        store_bf16x16(out + (size_t)row * kHid + n0 + cb, h);
     };
     auto sums = [&](int which, int cb, float (&h)[16]) {
         const float sum = column_sums16(h, lane);
@@ -366,37 +397,33 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const int cb = c_lo + 16 * i;
-        float v[16], dg[16], h[16];
-        tmem_ld16(d1 + lanes + cb, dg);
-        tmem_ld16(d0 + lanes + cb, v);
-        back(cb, v, dg, a.dz2, h);
-        put(n0 + cb, h);
+        float h[16];
+        back(d0, d1, cb, h);
+        put(H, n0 + cb, h);
+        put_peer(n0 + cb, h);
         sums(0, cb, h);
     }
     exchange();
     // dH1's own columns: dZ2 by W2's columns.
     mma_h(d1, idesc_back, [&](int c, int kk) { return sw128_desc_mn(w2b + c * kTile + kk * 2048, kMnBlock); });
+    store_half(a.dz2, H);
     if (tid < kTrN)
         part[kHid + n0 + tid] = (s_col[0][0][tid] + s_col[0][1][tid]) + (s_col[0][2][tid] + s_col[0][3][tid]);
-    float dg[2][16];
-#pragma unroll
-    for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            *reinterpret_cast<float4*>(&dg[i][4 * q]) =
-                reinterpret_cast<const float4*>(a.d1 + (size_t)row * kHid + n0 + c_lo + 16 * i)[q];
     ok = wait_commit(&bar, 0, a.err) && ok;
     tc_fence_after();
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const int cb = c_lo + 16 * i;
-        float v[16], h[16];
-        tmem_ld16(d1 + lanes + cb, v);
-        back(cb, v, dg[i], a.dz1, h);
+        float h[16];
+        back(d1, g1, cb, h);
+        put(w2f, n0 + cb, h);  // H may still be on its way out; layer 2's weights have done their work
         sums(1, cb, h);
     }
+    fence_proxy_async_smem();
     __syncthreads();
     if (tid < kTrN) part[n0 + tid] = (s_col[1][0][tid] + s_col[1][1][tid]) + (s_col[1][2][tid] + s_col[1][3][tid]);
+    store_half(a.dz1, w2f);
+    if (tid == 0) image_stores_done();
     tr_teardown<kRowTmem>(t.tmem);
 }
 
@@ -404,97 +431,100 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
 // (chunks of 64 as K; 512 rows up to a batch of 16,384: 128 blocks at 8192) for
 // a 128-row tile of a gradient.  Jobs 0-3: dW2's 128 x 128
 // quarters; 4, 5: dW1's halves; 6, 7: dW3 transposed ([256][16]), by halves.
-// Chunks stream through four stages.
+// One thread streams the chunks through four stages and issues the products.
+//
+// A partial sum is kept as the epilogue's threads have it: tiles of 16,384, in them
+// [column / 4][row][column % 4] (neighbouring lanes are neighbouring rows); dW3
+// after the six of them, in its own order.
 constexpr int kTrJobs = 8;
 constexpr uint32_t kTrSmem = kTrStages * 2 * kTile + 1024;
+constexpr uint32_t kTrTileSums = kBM * kTrN, kTrW3Sums = 6 * kTrTileSums;
+constexpr uint32_t kTrSums = kTrW3Sums + kOut * kHid;
+static_assert(kTrSums <= kParams, "a split's sums");
 
 __global__ void __launch_bounds__(kTrThreads) k_train_weights(const __grid_constant__ TrainArgs a) {
     extern __shared__ uint8_t raw[];
-    __shared__ uint64_t bars[kTrStages];
+    __shared__ uint64_t bars[2 * kTrStages + 1];  // a chunk has landed; has been used; all have been used
     __shared__ uint32_t slot;
+    __shared__ int s_ok;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int job = blockIdx.x;
-    const TrSetup t = tr_setup<kTrN>(raw, bars, kTrStages, &slot);
+    const TrSetup t = tr_setup<kTrN>(raw, bars, 2 * kTrStages + 1, &slot);
     griddep_wait();
     griddep_launch_dependents();
-    const int per = (int)(a.split_rows / kBK), c0 = (int)blockIdx.y * per, c1 = min(c0 + per, (int)(a.B / kBK));
+    const int per = (int)(a.split_rows / kBK), c0 = (int)blockIdx.y * per, n = min(per, (int)(a.B / kBK) - c0);
     float* const sums = a.weight_part + (size_t)blockIdx.y * kParams;
     const int mt = job < 4 ? job >> 1 : job & 1;
     const bool last_layer = job >= 6, first_layer = job == 4 || job == 5;
-    const __nv_bfloat16* A = (first_layer ? a.dz1 : (last_layer ? a.h2 : a.dz2)) + mt * kBM;
-    auto stage = [&](int c) {
-        const uint32_t sa = t.base + (uint32_t)((c - c0) & (kTrStages - 1)) * 2 * kTile, sb = sa + kTile;
-        const int r0 = c * kBK;
-        auto rows = [&](int r) { return r0 + r; };
-        stage_mn<kTrThreads>(sa, A, kHid, kBK, 0, 16, rows);
-        if (last_layer)
-            stage_mn<kTrThreads>(sb, a.dy, kOut, kBK, 0, 2, rows);
-        else if (first_layer)
-            stage_mn<kTrThreads>(sb, a.X, kInPad, kBK, 0, 16, [&](int r) { return a.n_rows ? a.idx[r0 + r] : (uint32_t)(r0 + r); });
-        else
-            stage_mn<kTrThreads>(sb, a.h1, kHid, kBK, (job & 1) * kTrN, 16, rows);
-    };
-    const uint32_t idesc = (last_layer ? idesc_bf16(kBM, kOut) : idesc_bf16(kBM, kTrN)) | kIdescAMn | kIdescBMn;
-    bool ok = true;
-    // Three chunks ahead; a commit group per chunk, empty ones past the end.
-    for (int c = c0; c < c0 + kTrStages - 1; ++c) {
-        if (c < c1) stage(c);
-        cp_async_commit_group();
-    }
-    for (int c = c0; c < c1; ++c) {
-        const int s = (c - c0) & (kTrStages - 1);
-        cp_async_wait<kTrStages - 2>();
-        fence_proxy_async_smem();
-        __syncthreads();
-        if (tid == 0) {
+    if (tid == 0) {
+        const uint8_t* A = first_layer ? a.dz1 : (last_layer ? a.h2 : a.dz2);
+        auto load = [&](int i) {  // chunk i of the split: half an image of each of an operand's 64-column blocks
+            const int s = i & (kTrStages - 1), c = c0 + i;
+            const uint32_t sa = t.base + (uint32_t)s * 2 * kTile, sb = sa + kTile;
+            const size_t image = (size_t)(c >> 1), half = (size_t)(c & 1) * kMnBlock;
+            mbar_arrive_expect_tx(&bars[s], 2 * kMnBlock + (last_layer ? kMnBlock : 2 * kMnBlock));
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                image_load(sa + b * kMnBlock, A + (image * 4 + 2 * mt + b) * kImage + half, kMnBlock, &bars[s]);
+                if (last_layer) {
+                    if (b == 0) image_load(sb, a.dy + image * kImage + half, kMnBlock, &bars[s]);
+                } else if (first_layer) {
+                    image_load(sb + b * kMnBlock, a.xt + (image * 2 + b) * kImage + half, kMnBlock, &bars[s]);
+                } else {
+                    image_load(sb + b * kMnBlock, a.h1 + (image * 4 + 2 * (job & 1) + b) * kImage + half, kMnBlock, &bars[s]);
+                }
+            }
+        };
+        const uint32_t idesc = (last_layer ? idesc_bf16(kBM, kOut) : idesc_bf16(kBM, kTrN)) | kIdescAMn | kIdescBMn;
+        bool ok = true;
+        for (int i = 0; i < min(n, kTrStages); ++i) load(i);
+        for (int i = 0; i < n; ++i) {
+            const int s = i & (kTrStages - 1);
+            ok = wait_commit(&bars[s], (i / kTrStages) & 1, a.err) && ok;
             tc_fence_after();
             const uint32_t sa = t.base + (uint32_t)s * 2 * kTile, sb = sa + kTile;
 #pragma unroll
             for (int kk = 0; kk < kBK / 16; ++kk)
                 umma_bf16(t.tmem, sw128_desc_mn(sa + kk * 2048, kMnBlock), sw128_desc_mn(sb + kk * 2048, kMnBlock), idesc,
-                          (c > c0 || kk > 0) ? 1u : 0u);
-            umma_commit(&bars[s]);
+                          (i > 0 || kk > 0) ? 1u : 0u);
+            umma_commit(&bars[kTrStages + s]);
+            // The stage of the chunk before this one, now that this one's products queue behind its.
+            const int next = i - 1 + kTrStages, before = (i - 1) & (kTrStages - 1);
+            if (i > 0 && next < n) {
+                ok = wait_commit(&bars[kTrStages + before], ((i - 1) / kTrStages) & 1, a.err) && ok;
+                load(next);
+            }
         }
-        // The stage that chunk c + 3 goes to was chunk c - 1's.
-        const int next = c + kTrStages - 1;
-        if (next < c1) {
-            if (c > c0) ok = wait_commit(&bars[(s + kTrStages - 1) & (kTrStages - 1)], ((c - 1 - c0) / kTrStages) & 1, a.err) && ok;
-            stage(next);
-        }
-        cp_async_commit_group();
+        s_ok = ok;
+        umma_commit(&bars[2 * kTrStages]);
     }
-    if (c1 > c0) {
-        const int l = c1 - 1 - c0;
-        ok = wait_commit(&bars[l & (kTrStages - 1)], (l / kTrStages) & 1, a.err) && ok;
-        tc_fence_after();
-        const int quarter = warp & 3, half = warp >> 2;
-        const int m = mt * kBM + quarter * 32 + lane;
-        const uint32_t t_lane = t.tmem + ((uint32_t)(quarter * 32) << 16);
-        if (last_layer) {
-            if (half == 0) {
-                float v[16];
-                tmem_ld16(t_lane, v);
+    __syncthreads();
+    const bool ok = wait_commit(&bars[2 * kTrStages], 0, a.err) && s_ok;
+    tc_fence_after();
+    const int quarter = warp & 3, half = warp >> 2, ml = quarter * 32 + lane;
+    const uint32_t t_lane = t.tmem + ((uint32_t)(quarter * 32) << 16);
+    if (last_layer) {
+        if (half == 0) {
+            float v[16];
+            tmem_ld16(t_lane, v);
 #pragma unroll
-                for (int i = 0; i < kOut; ++i) sums[kOffW3 + (size_t)i * kHid + m] = ok ? v[i] : 0.0f;
-            }
-        } else {
-            float* out = sums + (first_layer ? kOffW1 + (size_t)m * kInPad
-                                             : kOffW2 + (size_t)m * kHid + (job & 1) * kTrN);
+            for (int i = 0; i < kOut; ++i) sums[kTrW3Sums + (size_t)i * kHid + mt * kBM + ml] = ok ? v[i] : 0.0f;
+        }
+    } else {
+        float4* out = reinterpret_cast<float4*>(sums + (size_t)job * kTrTileSums);
 #pragma unroll 1
-            for (int cb = half * (kTrN / 2); cb < (half + 1) * (kTrN / 2); cb += 16) {
-                float v[16];
-                tmem_ld16(t_lane + cb, v);
+        for (int cb = half * (kTrN / 2); cb < (half + 1) * (kTrN / 2); cb += 16) {
+            float v[16];
+            tmem_ld16(t_lane + cb, v);
 #pragma unroll
-                for (int q = 0; q < 4; ++q)
-                    reinterpret_cast<float4*>(out + cb)[q] =
-                        ok ? make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3])
-                           : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
+            for (int q = 0; q < 4; ++q)
+                out[(cb / 4 + q) * kBM + ml] = ok ? make_float4(v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3])
+                                                  : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     }
     tr_teardown<kTrN>(t.tmem);
 }
-static_assert(kOffW1 % 4 == 0 && kOffW2 % 4 == 0 && kParams % 4 == 0, "four-wide stores");
+static_assert(kParams % 4 == 0, "four-wide stores");
 
 cudaError_t launch_forward_backward(const TrainArgs& a, cudaStream_t s) {
     if (a.B == 0 || a.B % kBM) return cudaErrorInvalidValue;
@@ -530,7 +560,8 @@ struct AdamArgs {
     __nv_bfloat16 *w1, *w2, *w3;
 };
 constexpr int kSumThreads = 256;
-constexpr int kSumBlocksW = (kParams + kSumThreads - 1) / kSumThreads;
+constexpr int kSumBlocksW = kTrSums / kSumThreads;
+static_assert(kTrSums % kSumThreads == 0, "a thread per weight");
 constexpr int kSumBlocksB = (kTrRowSums + kSumThreads / 32 - 1) / (kSumThreads / 32);
 
 template <bool ADAM>
@@ -542,10 +573,15 @@ __global__ void __launch_bounds__(kSumThreads) k_train_update(const __grid_const
     griddep_launch_dependents();
     float sum = 0.0f;
     if (blockIdx.x < (unsigned)kSumBlocksW) {
-        i = blockIdx.x * kSumThreads + threadIdx.x;
-        const bool weight = i < kOffB1 || (i >= kOffW2 && i < kOffB2) || (i >= kOffW3 && i < kOffB3);
-        if (!weight) return;
-        const float* part = a.weight_part + i;
+        const uint32_t j = blockIdx.x * kSumThreads + threadIdx.x;
+        const uint32_t tile = j / kTrTileSums, row = (j >> 2) & (kBM - 1), col = ((j >> 9) & 31u) * 4 + (j & 3u);
+        if (j >= kTrW3Sums)
+            i = kOffW3 + (j - kTrW3Sums);
+        else if (tile < 4)
+            i = kOffW2 + ((tile >> 1) * kBM + row) * kHid + (tile & 1) * kTrN + col;
+        else
+            i = kOffW1 + ((tile - 4) * kBM + row) * kInPad + col;
+        const float* part = a.weight_part + j;
         uint32_t q = 0;
         for (; q + 8 <= splits; q += 8) {  // eight in flight, added as a tree
             float t[8];

@@ -29,24 +29,23 @@ static void free_all(std::initializer_list<void*> ptrs) {
 static marl_status ensure_work(marl_surrogate* s, uint32_t B) {
     if (B <= s->work_b) return MARL_OK;
     cudaStreamSynchronize(s->stream);
-    free_all({s->xb, s->h1, s->h2, s->dy, s->dz2, s->dz1, s->tb, s->d1, s->y, s->idx, s->weight_part,
+    free_all({s->xb, s->h1, s->h2, s->dy, s->dz2, s->dz1, s->tb, s->y, s->xt, s->weight_part,
               s->row_part});
     s->weight_part = s->row_part = nullptr;
-    s->xb = s->h1 = s->h2 = s->dy = s->dz2 = s->dz1 = nullptr;
-    s->tb = s->d1 = s->y = nullptr;
-    s->idx = nullptr;
+    s->xb = nullptr;
+    s->tb = s->y = nullptr;
+    s->xt = s->h1 = s->h2 = s->dy = s->dz2 = s->dz1 = nullptr;
     s->work_b = 0;
     const size_t b = B;
     SCK(cudaMalloc((void**)&s->xb, b * mlp::kInPad * 2));
     SCK(cudaMalloc((void**)&s->h1, b * mlp::kHid * 2));
     SCK(cudaMalloc((void**)&s->h2, b * mlp::kHid * 2));
-    SCK(cudaMalloc((void**)&s->dy, b * mlp::kOut * 2));
+    SCK(cudaMalloc((void**)&s->dy, b * 128));
     SCK(cudaMalloc((void**)&s->dz2, b * mlp::kHid * 2));
     SCK(cudaMalloc((void**)&s->dz1, b * mlp::kHid * 2));
     SCK(cudaMalloc((void**)&s->tb, b * mlp::kOut * 4));
-    SCK(cudaMalloc((void**)&s->d1, b * mlp::kHid * 4));
     SCK(cudaMalloc((void**)&s->y, b * mlp::kOut * 4));
-    SCK(cudaMalloc((void**)&s->idx, b * 4));
+    SCK(cudaMalloc((void**)&s->xt, b * mlp::kInPad * 2));
     // A smaller batch may have as many partial sums (a split has at least 512 rows).
     const size_t splits = std::min<size_t>((b + 511) / 512, 32);
     SCK(cudaMalloc((void**)&s->weight_part, splits * mlp::kParams * 4));
@@ -95,9 +94,9 @@ static marl_status gemm(const mlp::GemmArgs& a, int bn, int epi, cudaStream_t st
 static mlp::TrainArgs train_args(marl_surrogate* s, uint32_t B, const __nv_bfloat16* X, const float* T,
                                  uint32_t n_rows, float* loss_sum) {
     mlp::TrainArgs a;
-    a.B = B, a.X = X, a.T = T, a.n_rows = n_rows, a.seed = s->cfg.seed, a.idx = s->idx;
+    a.B = B, a.X = X, a.T = T, a.n_rows = n_rows, a.seed = s->cfg.seed, a.xt = s->xt;
     a.w1 = s->w1, a.w2 = s->w2, a.w3 = s->w3, a.p = s->p;
-    a.h1 = s->h1, a.h2 = s->h2, a.dy = s->dy, a.dz2 = s->dz2, a.dz1 = s->dz1, a.d1 = s->d1, a.y = s->y;
+    a.h1 = s->h1, a.h2 = s->h2, a.dy = s->dy, a.dz2 = s->dz2, a.dz1 = s->dz1, a.y = s->y;
     a.split_rows = mlp::train_split_rows(B), a.weight_part = s->weight_part, a.row_part = s->row_part;
     a.g = s->g, a.loss_sum = loss_sum, a.err = s->d_err;
     return a;
@@ -168,7 +167,7 @@ void marl_surrogate_destroy(marl_surrogate* s) {
     if (!s) return;
     if (s->stream) cudaStreamSynchronize(s->stream);
     free_all({s->raw, s->X, s->T, s->norm, s->p, s->g, s->m, s->v, s->w1, s->w2, s->w3, s->xb, s->h1, s->h2, s->dy,
-              s->dz2, s->dz1, s->tb, s->d1, s->y, s->idx, s->weight_part, s->row_part, s->ih1, s->ih2, s->d_scalars, s->d_acc, s->d_err});
+              s->dz2, s->dz1, s->tb, s->y, s->xt, s->weight_part, s->row_part, s->ih1, s->ih2, s->d_scalars, s->d_acc, s->d_err});
     if (s->stream && s->own_stream) cudaStreamDestroy(s->stream);
     delete s;
 }

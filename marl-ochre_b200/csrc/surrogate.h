@@ -37,9 +37,9 @@ struct marl_surrogate {
 
     // Training work buffers for `work_b` rows.
     uint32_t work_b = 0;
-    __nv_bfloat16 *xb = nullptr, *h1 = nullptr, *h2 = nullptr, *dy = nullptr, *dz2 = nullptr, *dz1 = nullptr;
-    float *tb = nullptr, *d1 = nullptr, *y = nullptr;  // xb, tb: a caller's batch (gradients)
-    uint32_t* idx = nullptr;
+    __nv_bfloat16* xb = nullptr;  // xb, tb: a caller's batch (gradients)
+    float *tb = nullptr, *y = nullptr;
+    uint8_t *xt = nullptr, *h1 = nullptr, *h2 = nullptr, *dy = nullptr, *dz2 = nullptr, *dz1 = nullptr;  // tile images
     float *weight_part = nullptr, *row_part = nullptr;  // partial sums of the gradients and the loss
 
     // Inference work buffers for `infer_rows` rows.
