@@ -71,6 +71,13 @@ cudaError_t launch_mlp_fused(const FusedArgs& a, int num_sms, cudaStream_t s);
 // (bn, epi): (256, EPI_BIAS_GELU_FAST) or (16, EPI_BIAS_OUT).
 cudaError_t launch_gemm(const GemmArgs& a, int bn, int epi, cudaStream_t s);
 
+// The BF16 copies of the weights: row-major, and all of them as tile images.
+struct Bf16Weights {
+    __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr;
+    uint8_t* images = nullptr;  // kWeightImageBytes
+};
+constexpr uint32_t kWeightImageBytes = 2 * (kHid * kInPad + kHid * kHid + kOut * kHid);
+
 // One training step's buffers (B rows, a multiple of 128; see mlp_train.cu).
 struct TrainArgs {
     uint32_t B = 0;
@@ -78,7 +85,7 @@ struct TrainArgs {
     const float* T = nullptr;          // their targets [.][16]
     uint32_t n_rows = 0;               // batch row r is a hashed draw from [0, n_rows); 0: row r itself
     uint64_t seed = 0, step = 0;       // of the draws
-    const __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr;
+    const uint8_t* wi = nullptr;       // the BF16 weights' tile images
     const float* p = nullptr;          // FP32 parameters (the biases are read)
     // Images of 128-row, 64-column shared-memory tiles (16 KB, BF16): two to a row
     // tile of X, four of h1, h2, dz2 and dz1, one (16 columns used) of dy.
@@ -101,10 +108,8 @@ cudaError_t launch_forward_backward(const TrainArgs& a, cudaStream_t s);
 // FP32 parameters and their BF16 copies); both set *a.loss_sum.
 cudaError_t launch_train_gradients(const TrainArgs& a, cudaStream_t s);
 cudaError_t launch_train_update(const TrainArgs& a, float* p, float* m, float* v, float lr, float b1, float b2,
-                                float eps, uint64_t t, __nv_bfloat16* w1, __nv_bfloat16* w2, __nv_bfloat16* w3,
-                                cudaStream_t s);
-cudaError_t launch_weights_bf16(const float* p, __nv_bfloat16* w1, __nv_bfloat16* w2, __nv_bfloat16* w3,
-                                cudaStream_t s);
+                                float eps, uint64_t t, const Bf16Weights& w, cudaStream_t s);
+cudaError_t launch_weights_bf16(const float* p, const Bf16Weights& w, cudaStream_t s);
 cudaError_t launch_raw_stats(const float* raw, uint32_t n, double* acc, cudaStream_t s);
 cudaError_t launch_standardise(const float* raw, uint32_t n, const float* norm, __nv_bfloat16* X, float* T,
                                cudaStream_t s);

@@ -24,10 +24,11 @@
 // epilogues take gelu' from the tanh they have already taken, so the backward
 // ones take none.  The batch is never copied: its rows are drawn by the loads that
 // use them.
-// A step takes 37 us at a batch of 8192 (35 at 512, 221 at 65,536).  With rows
-// written and read 16 bytes a thread instead of tile images it took 54 (50, 335),
-// with a kernel per layer and direction 71 (55, 372), as 14 kernels with transposed
-// copies and shared-memory atomics in the loss 347 at 8192.
+// A step takes 34 us at a batch of 8192 (31 at 512, 201 at 65,536).  With weights
+// gathered 16 bytes a thread and a wait of the block pair before each overwrite it
+// took 37 (34, 220), with rows instead of tile images 54 (50, 335), with a kernel
+// per layer and direction 71 (55, 372), as 14 kernels with transposed copies and
+// shared-memory atomics in the loss 347 at 8192.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -59,18 +60,6 @@ __device__ __forceinline__ void stage_k(uint32_t dst, const __nv_bfloat16* src, 
     for (int p = threadIdx.x; p < rows * pieces; p += THREADS) {
         const int r = p / pieces, q = p % pieces;
         cp_async16_zfill(dst + r * 128 + ((q ^ (r & 7)) << 4), src + (size_t)at(r) * ld + k0 + q * 8, 16u);
-    }
-}
-
-// Rows at(0..krows-1) of a row-major matrix as k, columns n0 .. n0 + 8 pieces - 1
-// as the operand's M or N: MN-major, blocks of 64 columns.
-template <int THREADS, class At>
-__device__ __forceinline__ void stage_mn(uint32_t dst, const __nv_bfloat16* src, int ld, int krows, int n0, int pieces,
-                                         At at) {
-    for (int p = threadIdx.x; p < krows * pieces; p += THREADS) {
-        const int r = p / pieces, q = p % pieces;
-        cp_async16_zfill(dst + (q >> 3) * kMnBlock + r * 128 + (((q & 7) ^ (r & 7)) << 4),
-                         src + (size_t)at(r) * ld + n0 + q * 8, 16u);
     }
 }
 
@@ -131,7 +120,7 @@ __device__ __forceinline__ uint32_t drawn_row(const TrainArgs& a, uint32_t r) {
 // backward.  A cluster of two blocks owns 128 rows; each block computes 128 of a
 // layer's 256 columns, so that 8192 rows are 128 blocks, and writes what the next
 // layer reads (H1, then H2, then dZ2) into both blocks' shared memory.  The
-// weights it needs are all staged at the start, and gelu' of layers 1 and 2 stays
+// weights it needs are fetched once, in the order of their use, and gelu' of layers 1 and 2 stays
 // in tensor memory.  What the weight gradients need leaves as images of the
 // shared-memory tiles (128 rows of 64 columns, swizzled, 16 KB), one bulk copy
 // each: k_train_weights loads halves of them (64 rows) the same way, and they are
@@ -142,9 +131,11 @@ __device__ __forceinline__ uint32_t drawn_row(const TrainArgs& a, uint32_t r) {
 // 32 (w / 4).. of its block's 128.
 constexpr int kRowThreads = 512;
 constexpr uint32_t kRowTmem = 512;              // columns 0-127 and 128-255: an accumulator each; 256-383: gelu' of layer 1
-constexpr uint32_t kRowW2F = 0;                 // W2's own rows, K-major (forward), four chunks of 64 k
-constexpr uint32_t kRowW2B = 4 * kTile;         // W2's own columns, MN-major (backward), likewise
-constexpr uint32_t kRowH = 8 * kTile;           // X and W1, then H1, H2, dZ2: four chunks of 64 k
+// Shared memory, each four chunks of 64 k.  What is written next goes where both
+// blocks have finished by the exchange before it, so nothing else has to be waited for.
+constexpr uint32_t kRowP = 0;                   // X and W1, then H2, then dZ1
+constexpr uint32_t kRowQ = 4 * kTile;           // H1, then dZ2
+constexpr uint32_t kRowW2 = 8 * kTile;          // W2's own rows (K-major), then its own columns (MN-major)
 constexpr uint32_t kRowW3 = 12 * kTile;         // four chunks [16][64]: K-major forward, MN-major backward
 constexpr uint32_t kRowW3Chunk = kOut * 128;
 constexpr uint32_t kRowDy = kRowW3 + 4 * kRowW3Chunk;
@@ -179,7 +170,7 @@ __device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.pr
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
     k_train_rows(const __grid_constant__ TrainArgs a) {
     extern __shared__ uint8_t raw[];
-    __shared__ uint64_t bar;
+    __shared__ uint64_t bars[5];
     __shared__ uint32_t slot;
     __shared__ uint32_t s_idx[kBM];
     __shared__ float s_col[2][4][kTrN], s_col3[4][kOut], s_b1[kTrN], s_b2[kTrN], s_b3[kOut], s_loss[4];
@@ -187,99 +178,97 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
     const uint32_t rank = blockIdx.x & 1u;
     const uint32_t tile = blockIdx.x >> 1;
     const int m0 = (int)tile * kBM, n0 = (int)rank * kTrN;
-    const TrSetup t = tr_setup<kRowTmem>(raw, &bar, 1, &slot);
-    const uint32_t w2f = t.base + kRowW2F, w2b = t.base + kRowW2B, H = t.base + kRowH, w3 = t.base + kRowW3,
-                   dy = t.base + kRowDy, peer = cluster_map(H, rank ^ 1u);
+    const TrSetup t = tr_setup<kRowTmem>(raw, bars, 5, &slot);
+    uint64_t &bar = bars[0], *const w_bar = bars + 1;  // products done; W1, W2's rows, W3, W2's columns have landed
+    const uint32_t P = t.base + kRowP, Q = t.base + kRowQ, w2 = t.base + kRowW2, w3 = t.base + kRowW3,
+                   dy = t.base + kRowDy, peer = cluster_map(t.base, rank ^ 1u) - t.base;
+    cluster_arrive();  // this block has started: its shared memory may be written
     if (tid < kBM) s_idx[tid] = drawn_row(a, (uint32_t)(m0 + tid));
+    __syncthreads();
     griddep_wait();  // Adam's weights
     griddep_launch_dependents();
-    if (tid < kTrN) s_b1[tid] = a.p[kOffB1 + n0 + tid], s_b2[tid] = a.p[kOffB2 + n0 + tid];
-    if (tid < kOut) s_b3[tid] = a.p[kOffB3 + tid];
-    __syncthreads();
-    auto self = [](int r) { return r; };
+    if (tid == 0) {
+        mbar_arrive_expect_tx(&w_bar[0], 2 * kTile);
+        image_load(P + 2 * kTile, a.wi + rank * 2 * kImage, 2 * kTile, &w_bar[0]);
+    }
+    // X is gathered, a commit group per chunk.
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-        stage_k<kRowThreads>(H + c * kTile, a.X, kInPad, kBM, c * kBK, 8, [&](int r) { return s_idx[r]; });
-        stage_k<kRowThreads>(H + (2 + c) * kTile, a.w1 + (size_t)n0 * kInPad, kInPad, kTrN, c * kBK, 8, self);
+        stage_k<kRowThreads>(P + c * kTile, a.X, kInPad, kBM, c * kBK, 8, [&](int r) { return s_idx[r]; });
         cp_async_commit_group();
     }
-#pragma unroll
-    for (int c = 0; c < 4; ++c)
-        stage_k<kRowThreads>(w2f + c * kTile, a.w2 + (size_t)n0 * kHid, kHid, kTrN, c * kBK, 8, self);
-    cp_async_commit_group();
-#pragma unroll
-    for (int c = 0; c < 4; ++c) {
-        stage_k<kRowThreads>(w3 + c * kRowW3Chunk, a.w3, kHid, kOut, c * kBK, 8, self);
-        stage_mn<kRowThreads>(w2b + c * kTile, a.w2 + (size_t)c * kBK * kHid, kHid, kBK, n0, 16, self);
+    if (tid == 0) {
+        mbar_arrive_expect_tx(&w_bar[1], 4 * kTile);
+        image_load(w2, a.wi + (4 + rank * 4) * kImage, 4 * kTile, &w_bar[1]);
+        mbar_arrive_expect_tx(&w_bar[2], 4 * kRowW3Chunk);
+        image_load(w3, a.wi + 12 * kImage, 4 * kRowW3Chunk, &w_bar[2]);
     }
-    cp_async_commit_group();
+    if (tid < kTrN) s_b1[tid] = a.p[kOffB1 + n0 + tid], s_b2[tid] = a.p[kOffB2 + n0 + tid];
+    if (tid < kOut) s_b3[tid] = a.p[kOffB3 + tid];
 
     const uint32_t d0 = t.tmem, d1 = t.tmem + kTrN, g1 = t.tmem + 2 * kTrN;  // the accumulators, gelu'
     const uint32_t idesc = idesc_bf16(kBM, kTrN), idesc_back = idesc | kIdescBMn;
     // Layer 1: X (128 k) by W1's own rows.
 #pragma unroll
     for (int c = 0; c < 2; ++c) {
-        if (c == 0) cp_async_wait<3>();
-        else cp_async_wait<2>();
+        if (c == 0) cp_async_wait<1>();
+        else cp_async_wait<0>();
         fence_proxy_async_smem();
         __syncthreads();
         if (tid == 0) {
+            if (c == 0) wait_commit(&w_bar[0], 0, a.err);
             tc_fence_after();
 #pragma unroll
             for (int kk = 0; kk < 4; ++kk)
-                umma_bf16(d0, sw128_desc(H + c * kTile + kk * 32), sw128_desc(H + (2 + c) * kTile + kk * 32), idesc,
+                umma_bf16(d0, sw128_desc(P + c * kTile + kk * 32), sw128_desc(P + (2 + c) * kTile + kk * 32), idesc,
                           (c > 0 || kk > 0) ? 1u : 0u);
             if (c == 1) umma_commit(&bar);
-            if (c == (int)rank) image_store(a.xt + ((size_t)tile * 2 + c) * kImage, H + c * kTile, kTile);
+            if (c == (int)rank) image_store(a.xt + ((size_t)tile * 2 + c) * kImage, P + c * kTile, kTile);
         }
     }
     bool ok = wait_commit(&bar, 0, a.err);
     tc_fence_after();
-    if (tid == 0) image_stores_read();
-    cluster_arrive();
-    cluster_wait();  // neither block reads X or W1 any more: H1 may take their place
+    cluster_wait();
 
     const int quarter = warp & 3, c_lo = (warp >> 2) * 32;
     const int rl = quarter * 32 + lane;
     const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
-    // 16 columns (from column `col` of 256) of this thread's row into an image of
-    // four chunks, or into the peer's H.
-    auto pieces = [&](int col, const float (&h)[16], auto store) {
-        const uint32_t at = (uint32_t)(col >> 6) * kTile + (uint32_t)rl * 128, q = (uint32_t)(col & 63) >> 3;
+    // 16 columns (from column `col` of 256) of this thread's row into the operand at
+    // `to`, here and, where the next product needs all 256, in the other block.
+    auto put = [&](uint32_t to, int col, const float (&h)[16], bool both) {
+        to += (uint32_t)(col >> 6) * kTile + (uint32_t)rl * 128;
+        const uint32_t q = (uint32_t)(col & 63) >> 3;
 #pragma unroll
-        for (uint32_t i = 0; i < 2; ++i)
-            store(at + (((q + i) ^ ((uint32_t)rl & 7u)) << 4),
-                  make_uint4(pack_bf16(h[8 * i], h[8 * i + 1]), pack_bf16(h[8 * i + 2], h[8 * i + 3]),
-                             pack_bf16(h[8 * i + 4], h[8 * i + 5]), pack_bf16(h[8 * i + 6], h[8 * i + 7])));
-    };
-    auto put = [&](uint32_t image, int col, const float (&h)[16]) {
-        pieces(col, h, [&](uint32_t at, uint4 v) {
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(image + at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+        for (uint32_t i = 0; i < 2; ++i) {
+            const uint4 v = make_uint4(pack_bf16(h[8 * i], h[8 * i + 1]), pack_bf16(h[8 * i + 2], h[8 * i + 3]),
+                                       pack_bf16(h[8 * i + 4], h[8 * i + 5]), pack_bf16(h[8 * i + 6], h[8 * i + 7]));
+            const uint32_t at = to + (((q + i) ^ ((uint32_t)rl & 7u)) << 4);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
                          : "memory");
-        });
+            if (both) cluster_store(at + peer, v);
+        }
     };
-    auto put_peer = [&](int col, const float (&h)[16]) {
-        pieces(col, h, [&](uint32_t at, uint4 v) { cluster_store(peer + at, v); });
-    };
-    // This block's half of an image in H (or at `from`) to memory.
+    // This block's half of an operand to memory.
     auto store_half = [&](uint8_t* images, uint32_t from) {
         if (tid == 0) image_store(images + ((size_t)tile * 4 + 2 * rank) * kImage, from + 2 * rank * kTile, 2 * kTile);
     };
-    // After it, both blocks have written H.
+    // Before it, what both blocks have written, sent and had multiplied; after it, what uses that.
     auto exchange = [&]() {
+        if (tid == 0) image_stores_read();
         fence_proxy_async_all();
         tc_fence_before();
         cluster_arrive();
         cluster_wait();
     };
-    // D = H (256 k) by B's chunks.
-    auto mma_h = [&](uint32_t d, uint32_t idesc_n, auto bdesc) {
+    // D = A (256 k) by B's chunks.
+    auto mma = [&](uint32_t d, uint32_t A, uint32_t idesc_n, uint64_t* landed, auto bdesc) {
         if (tid == 0) {
+            wait_commit(landed, 0, a.err);
             fence_proxy_async_all();
             tc_fence_after();
 #pragma unroll
             for (int k = 0; k < 16; ++k)
-                umma_bf16(d, sw128_desc(H + (k >> 2) * kTile + (k & 3) * 32), bdesc(k >> 2, k & 3), idesc_n, k > 0 ? 1u : 0u);
+                umma_bf16(d, sw128_desc(A + (k >> 2) * kTile + (k & 3) * 32), bdesc(k >> 2, k & 3), idesc_n, k > 0 ? 1u : 0u);
             umma_commit(&bar);
         }
     };
@@ -294,20 +283,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
 #pragma unroll
         for (int j = 0; j < 16; ++j) g[j] = __float_as_uint(v[j]);
         tmem_st16(g1 + lanes + cb, g);
-        put(H, n0 + cb, h);
-        put_peer(n0 + cb, h);
+        put(Q, n0 + cb, h, true);
     }
     tmem_st_wait();
-    cp_async_wait<1>();
     exchange();
     // Layer 2: H1 by W2's own rows.
-    mma_h(d1, idesc, [&](int c, int kk) { return sw128_desc(w2f + c * kTile + kk * 32); });
-    store_half(a.h1, H);
+    mma(d1, Q, idesc, &w_bar[1], [&](int c, int kk) { return sw128_desc(w2 + c * kTile + kk * 32); });
+    store_half(a.h1, Q);
     ok = wait_commit(&bar, 1, a.err) && ok;
     tc_fence_after();
-    if (tid == 0) image_stores_read();
-    cluster_arrive();
-    cluster_wait();  // neither block reads H1 any more
+    if (tid == 0) {  // W2's own columns, chunk c: its rows 64 c.., a half of two row images
+        mbar_arrive_expect_tx(&w_bar[3], 4 * kTile);
+#pragma unroll 1
+        for (uint32_t c = 0; c < 4; ++c)
+#pragma unroll
+            for (uint32_t b = 0; b < 2; ++b)
+                image_load(w2 + c * kTile + b * kMnBlock,
+                           a.wi + (4 + (c >> 1) * 4 + 2 * rank + b) * kImage + (c & 1) * kMnBlock, kMnBlock, &w_bar[3]);
+    }
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
         const int cb = c_lo + 16 * i;
@@ -321,29 +314,29 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
             g[j] = __float_as_uint(grad);
         }
         tmem_st16(d1 + lanes + cb, g);
-        put(H, n0 + cb, h);
-        put_peer(n0 + cb, h);
+        put(P, n0 + cb, h, true);
     }
     tmem_st_wait();
-    cp_async_wait<0>();
     exchange();
     // Layer 3 and the loss, in both blocks alike; the first one writes them.
-    mma_h(d0, idesc_bf16(kBM, kOut), [&](int c, int kk) { return sw128_desc(w3 + c * kRowW3Chunk + kk * 32); });
-    store_half(a.h2, H);
+    mma(d0, P, idesc_bf16(kBM, kOut), &w_bar[2], [&](int c, int kk) { return sw128_desc(w3 + c * kRowW3Chunk + kk * 32); });
+    store_half(a.h2, P);
+    float4 target[4];
+    if (warp < 4) {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) target[q] = reinterpret_cast<const float4*>(a.T + (size_t)s_idx[rl] * kOut)[q];
+    }
     ok = wait_commit(&bar, 0, a.err) && ok;
     tc_fence_after();
-    if (tid == 0) image_stores_read();
-    cluster_arrive();  // this block reads H2 no more; waited for before dZ2 takes its place
     if (warp < 4) {
         float v[16], g[16];
         tmem_ld16(d0 + lanes, v);
-        const float4* tp = reinterpret_cast<const float4*>(a.T + (size_t)s_idx[rl] * kOut);
         float4* yp = reinterpret_cast<float4*>(a.y + (size_t)(m0 + rl) * kOut);
         const float sc = 2.0f / ((float)a.B * 16.0f);
         float loss = 0.0f;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-            const float4 tt = tp[q];
+            const float4 tt = target[q];
             const float y0 = v[4 * q] + s_b3[4 * q], y1 = v[4 * q + 1] + s_b3[4 * q + 1],
                         y2 = v[4 * q + 2] + s_b3[4 * q + 2], y3 = v[4 * q + 3] + s_b3[4 * q + 3];
             const float e0 = y0 - tt.x, e1 = y1 - tt.y, e2 = y2 - tt.z, e3 = y3 - tt.w;
@@ -381,7 +374,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
     if (rank == 0 && tid == kOut) part[2 * kHid + kOut] = (s_loss[0] + s_loss[1]) + (s_loss[2] + s_loss[3]);
     ok = wait_commit(&bar, 1, a.err) && ok;
     tc_fence_after();
-    cluster_wait();
     // dZ = dH gelu'.
     auto back = [&](uint32_t d, uint32_t g, int cb, float (&h)[16]) {
         float v[16], dg[16];
@@ -399,14 +391,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
         const int cb = c_lo + 16 * i;
         float h[16];
         back(d0, d1, cb, h);
-        put(H, n0 + cb, h);
-        put_peer(n0 + cb, h);
+        put(Q, n0 + cb, h, true);
         sums(0, cb, h);
     }
     exchange();
     // dH1's own columns: dZ2 by W2's columns.
-    mma_h(d1, idesc_back, [&](int c, int kk) { return sw128_desc_mn(w2b + c * kTile + kk * 2048, kMnBlock); });
-    store_half(a.dz2, H);
+    mma(d1, Q, idesc_back, &w_bar[3], [&](int c, int kk) { return sw128_desc_mn(w2 + c * kTile + kk * 2048, kMnBlock); });
+    store_half(a.dz2, Q);
     if (tid < kTrN)
         part[kHid + n0 + tid] = (s_col[0][0][tid] + s_col[0][1][tid]) + (s_col[0][2][tid] + s_col[0][3][tid]);
     ok = wait_commit(&bar, 0, a.err) && ok;
@@ -416,13 +407,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
         const int cb = c_lo + 16 * i;
         float h[16];
         back(d1, g1, cb, h);
-        put(w2f, n0 + cb, h);  // H may still be on its way out; layer 2's weights have done their work
+        put(P, n0 + cb, h, false);
         sums(1, cb, h);
     }
     fence_proxy_async_smem();
     __syncthreads();
     if (tid < kTrN) part[n0 + tid] = (s_col[1][0][tid] + s_col[1][1][tid]) + (s_col[1][2][tid] + s_col[1][3][tid]);
-    store_half(a.dz1, w2f);
+    store_half(a.dz1, P);
     if (tid == 0) image_stores_done();
     tr_teardown<kRowTmem>(t.tmem);
 }
@@ -540,16 +531,33 @@ cudaError_t launch_forward_backward(const TrainArgs& a, cudaStream_t s) {
 }
 
 // ------------------------------------------------- gradients and Adam ----
-// The BF16 copies of the parameters that the tensor cores read.
-__device__ __forceinline__ void put_bf16(uint32_t i, float v, __nv_bfloat16* w1, __nv_bfloat16* w2, __nv_bfloat16* w3) {
-    const __nv_bfloat16 b = __float2bfloat16_rn(v);
-    if (i < kOffB1)
-        w1[i] = b;
-    else if (i >= kOffW2 && i < kOffB2)
-        w2[i - kOffW2] = b;
-    else if (i >= kOffW3 && i < kOffB3)
-        w3[i - kOffW3] = b;
+// The BF16 copies of the parameters that the tensor cores read: row-major for
+// inference, as tile images (row n, column k) for training: W1's four (rows 128,
+// columns 64 each), W2's eight, W3's columns in four of 16 rows.
+__device__ __forceinline__ uint32_t image_at(uint32_t n, uint32_t k) {
+    return n * 128 + ((((k & 63u) >> 3) ^ (n & 7u)) << 4) + (k & 7u) * 2;
 }
+__device__ __forceinline__ void put_bf16(uint32_t i, float v, const Bf16Weights& w) {
+    const __nv_bfloat16 b = __float2bfloat16_rn(v);
+    uint32_t at;
+    if (i < kOffB1) {
+        const uint32_t n = i / kInPad, k = i % kInPad;
+        w.w1[i] = b;
+        at = ((n >> 7) * 2 + (k >> 6)) * kImage + image_at(n & 127u, k);
+    } else if (i >= kOffW2 && i < kOffB2) {
+        const uint32_t j = i - kOffW2, n = j / kHid, k = j % kHid;
+        w.w2[j] = b;
+        at = (4 + (n >> 7) * 4 + (k >> 6)) * kImage + image_at(n & 127u, k);
+    } else if (i >= kOffW3 && i < kOffB3) {
+        const uint32_t j = i - kOffW3, n = j / kHid, k = j % kHid;
+        w.w3[j] = b;
+        at = 12 * kImage + (k >> 6) * kRowW3Chunk + image_at(n, k);
+    } else {
+        return;
+    }
+    *reinterpret_cast<__nv_bfloat16*>(w.images + at) = b;
+}
+static_assert(12 * kImage + 4 * kRowW3Chunk == kWeightImageBytes, "the weights' images");
 
 // Adds the partial sums of gradient i (thread i for a weight, a warp for each of
 // the 528 biases and the loss) in a fixed order and, with ADAM, updates the FP32
@@ -557,7 +565,7 @@ __device__ __forceinline__ void put_bf16(uint32_t i, float v, __nv_bfloat16* w1,
 struct AdamArgs {
     float *p, *m, *v;
     float lr, b1, b2, eps, bc1, bc2;
-    __nv_bfloat16 *w1, *w2, *w3;
+    Bf16Weights w;
 };
 constexpr int kSumThreads = 256;
 constexpr int kSumBlocksW = kTrSums / kSumThreads;
@@ -613,25 +621,23 @@ __global__ void __launch_bounds__(kSumThreads) k_train_update(const __grid_const
         o.v[i] = vi;
         const float pi = o.p[i] - o.lr * (mi / o.bc1) / (sqrtf(vi / o.bc2) + o.eps);
         o.p[i] = pi;
-        put_bf16(i, pi, o.w1, o.w2, o.w3);
+        put_bf16(i, pi, o.w);
     } else {
         a.g[i] = gi;
     }
 }
 
-__global__ void k_weights_bf16(const float* __restrict__ p, __nv_bfloat16* __restrict__ w1,
-                               __nv_bfloat16* __restrict__ w2, __nv_bfloat16* __restrict__ w3) {
+__global__ void k_weights_bf16(const float* __restrict__ p, Bf16Weights w) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < kParams; i += gridDim.x * blockDim.x)
-        put_bf16(i, p[i], w1, w2, w3);
+        put_bf16(i, p[i], w);
 }
 
 cudaError_t launch_train_update(const TrainArgs& a, float* p, float* m, float* v, float lr, float b1, float b2,
-                                float eps, uint64_t t, __nv_bfloat16* w1, __nv_bfloat16* w2, __nv_bfloat16* w3,
-                                cudaStream_t s) {
+                                float eps, uint64_t t, const Bf16Weights& w, cudaStream_t s) {
     const float bc1 = 1.0f - (float)pow((double)b1, (double)t);
     const float bc2 = 1.0f - (float)pow((double)b2, (double)t);
     return launch_dependent(k_train_update<true>, dim3(kSumBlocksW + kSumBlocksB), dim3(kSumThreads), 0, s, a,
-                            AdamArgs{p, m, v, lr, b1, b2, eps, bc1, bc2, w1, w2, w3}, train_splits(a.B, a.split_rows));
+                            AdamArgs{p, m, v, lr, b1, b2, eps, bc1, bc2, w}, train_splits(a.B, a.split_rows));
 }
 
 cudaError_t launch_train_gradients(const TrainArgs& a, cudaStream_t s) {
@@ -639,9 +645,8 @@ cudaError_t launch_train_gradients(const TrainArgs& a, cudaStream_t s) {
                             AdamArgs{}, train_splits(a.B, a.split_rows));
 }
 
-cudaError_t launch_weights_bf16(const float* p, __nv_bfloat16* w1, __nv_bfloat16* w2, __nv_bfloat16* w3,
-                                cudaStream_t s) {
-    k_weights_bf16<<<256, 256, 0, s>>>(p, w1, w2, w3);
+cudaError_t launch_weights_bf16(const float* p, const Bf16Weights& w, cudaStream_t s) {
+    k_weights_bf16<<<256, 256, 0, s>>>(p, w);
     return cudaGetLastError();
 }
 

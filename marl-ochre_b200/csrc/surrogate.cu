@@ -26,6 +26,8 @@ static void free_all(std::initializer_list<void*> ptrs) {
         if (p) cudaFree(p);
 }
 
+static mlp::Bf16Weights bf16_weights(const marl_surrogate* s) { return {s->w1, s->w2, s->w3, s->wi}; }
+
 static marl_status ensure_work(marl_surrogate* s, uint32_t B) {
     if (B <= s->work_b) return MARL_OK;
     cudaStreamSynchronize(s->stream);
@@ -95,7 +97,7 @@ static mlp::TrainArgs train_args(marl_surrogate* s, uint32_t B, const __nv_bfloa
                                  uint32_t n_rows, float* loss_sum) {
     mlp::TrainArgs a;
     a.B = B, a.X = X, a.T = T, a.n_rows = n_rows, a.seed = s->cfg.seed, a.xt = s->xt;
-    a.w1 = s->w1, a.w2 = s->w2, a.w3 = s->w3, a.p = s->p;
+    a.wi = s->wi, a.p = s->p;
     a.h1 = s->h1, a.h2 = s->h2, a.dy = s->dy, a.dz2 = s->dz2, a.dz1 = s->dz1, a.y = s->y;
     a.split_rows = mlp::train_split_rows(B), a.weight_part = s->weight_part, a.row_part = s->row_part;
     a.g = s->g, a.loss_sum = loss_sum, a.err = s->d_err;
@@ -166,7 +168,7 @@ marl_status marl_surrogate_config_default(marl_surrogate_config* c) {
 void marl_surrogate_destroy(marl_surrogate* s) {
     if (!s) return;
     if (s->stream) cudaStreamSynchronize(s->stream);
-    free_all({s->raw, s->X, s->T, s->norm, s->p, s->g, s->m, s->v, s->w1, s->w2, s->w3, s->xb, s->h1, s->h2, s->dy,
+    free_all({s->raw, s->X, s->T, s->norm, s->p, s->g, s->m, s->v, s->w1, s->w2, s->w3, s->wi, s->xb, s->h1, s->h2, s->dy,
               s->dz2, s->dz1, s->tb, s->y, s->xt, s->weight_part, s->row_part, s->ih1, s->ih2, s->d_scalars, s->d_acc, s->d_err});
     if (s->stream && s->own_stream) cudaStreamDestroy(s->stream);
     delete s;
@@ -199,6 +201,7 @@ marl_status marl_surrogate_create(const marl_surrogate_config* cfg, marl_surroga
     if ((e = cudaMalloc((void**)&s->w1, (size_t)mlp::kHid * mlp::kInPad * 2)) ||
         (e = cudaMalloc((void**)&s->w2, (size_t)mlp::kHid * mlp::kHid * 2)) ||
         (e = cudaMalloc((void**)&s->w3, (size_t)mlp::kOut * mlp::kHid * 2)) ||
+        (e = cudaMalloc((void**)&s->wi, mlp::kWeightImageBytes)) ||
         (e = cudaMalloc((void**)&s->norm, MARL_SURR_NORM * 4)) || (e = cudaMalloc((void**)&s->d_acc, 256 * 8)) ||
         (e = cudaMalloc((void**)&s->d_err, 16)))
         return bad(e, "surrogate buffers");
@@ -206,7 +209,7 @@ marl_status marl_surrogate_create(const marl_surrogate_config* cfg, marl_surroga
     cudaMemsetAsync(s->v, 0, P * 4, s->stream);
     cudaMemsetAsync(s->d_err, 0, 16, s->stream);
     if ((e = mlp::launch_init_weights(s->p, cfg->seed, s->stream))) return bad(e, "init weights");
-    if ((e = mlp::launch_weights_bf16(s->p, s->w1, s->w2, s->w3, s->stream))) return bad(e, "bf16 weights");
+    if ((e = mlp::launch_weights_bf16(s->p, bf16_weights(s), s->stream))) return bad(e, "bf16 weights");
     if ((e = cudaStreamSynchronize(s->stream))) return bad(e, "surrogate create");
     *out = s;
     return MARL_OK;
@@ -305,7 +308,7 @@ marl_status marl_surrogate_train(marl_surrogate* s, uint32_t steps, float* loss_
         SCK(mlp::launch_forward_backward(a, cs));
         ++s->adam_t;
         SCK(mlp::launch_train_update(a, s->p, s->m, s->v, s->cfg.lr, s->cfg.beta1, s->cfg.beta2, s->cfg.adam_eps,
-                                     s->adam_t, s->w1, s->w2, s->w3, cs));
+                                     s->adam_t, bf16_weights(s), cs));
     }
     if (loss_out) {
         SCK(cudaMemcpyAsync(loss_out, s->d_scalars, (size_t)steps * 4, cudaMemcpyDeviceToHost, cs));
@@ -384,7 +387,7 @@ marl_status marl_surrogate_set_weights(marl_surrogate* s, const float* params, c
     // Ordered on the surrogate's stream, ahead of the kernels that read them.
     if (params) {
         SCK(cudaMemcpyAsync(s->p, params, (size_t)mlp::kParams * 4, cudaMemcpyHostToDevice, s->stream));
-        SCK(mlp::launch_weights_bf16(s->p, s->w1, s->w2, s->w3, s->stream));
+        SCK(mlp::launch_weights_bf16(s->p, bf16_weights(s), s->stream));
     }
     if (norm) {
         std::memcpy(s->h_norm, norm, sizeof(s->h_norm));

@@ -32,6 +32,7 @@ struct marl_surrogate {
     float* m = nullptr;  // Adam moments
     float* v = nullptr;
     __nv_bfloat16 *w1 = nullptr, *w2 = nullptr, *w3 = nullptr;
+    uint8_t* wi = nullptr;  // the same as tile images (training)
     uint64_t adam_t = 0;
     uint64_t batches = 0;  // batch counter (sampling stream)
 
