@@ -24,7 +24,8 @@
 // epilogues take gelu' from the tanh they have already taken, so the backward
 // ones take none.  The batch is never copied: its rows are drawn by the loads that
 // use them.
-// A step takes 34 us at a batch of 8192 (31 at 512, 201 at 65,536).  With weights
+// A step takes 32 us at a batch of 8192 (30 at 512, 200 at 65,536).  With X and the
+// moments read after the wait for the kernel before it took 34 (31, 201), with weights
 // gathered 16 bytes a thread and a wait of the block pair before each overwrite it
 // took 37 (34, 220), with rows instead of tile images 54 (50, 335), with a kernel
 // per layer and direction 71 (55, 372), as 14 kernels with transposed copies and
@@ -185,17 +186,19 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
     cluster_arrive();  // this block has started: its shared memory may be written
     if (tid < kBM) s_idx[tid] = drawn_row(a, (uint32_t)(m0 + tid));
     __syncthreads();
+    // X is gathered, a commit group per chunk, before the wait: no kernel that may
+    // still be running writes it (whoever does ends with a synchronisation, or is a
+    // copy, which this kernel does not overtake).
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+        stage_k<kRowThreads>(P + c * kTile, a.X, kInPad, kBM, c * kBK, 8, [&](int r) { return s_idx[r]; });
+        cp_async_commit_group();
+    }
     griddep_wait();  // Adam's weights
     griddep_launch_dependents();
     if (tid == 0) {
         mbar_arrive_expect_tx(&w_bar[0], 2 * kTile);
         image_load(P + 2 * kTile, a.wi + rank * 2 * kImage, 2 * kTile, &w_bar[0]);
-    }
-    // X is gathered, a commit group per chunk.
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {
-        stage_k<kRowThreads>(P + c * kTile, a.X, kInPad, kBM, c * kBK, 8, [&](int r) { return s_idx[r]; });
-        cp_async_commit_group();
     }
     if (tid == 0) {
         mbar_arrive_expect_tx(&w_bar[1], 4 * kTile);
@@ -577,9 +580,12 @@ __global__ void __launch_bounds__(kSumThreads) k_train_update(const __grid_const
                                                               uint32_t splits) {
     uint32_t i;
     bool owner = true;
-    griddep_wait();
-    griddep_launch_dependents();
-    float sum = 0.0f;
+    float sum = 0.0f, m0 = 0.0f, v0 = 0.0f, p0 = 0.0f;
+    // Read ahead of the wait: the step before, which wrote them, was over before this
+    // step's row kernel went past its own.
+    auto moments = [&]() {
+        if constexpr (ADAM) m0 = __ldcg(o.m + i), v0 = __ldcg(o.v + i), p0 = __ldcg(o.p + i);
+    };
     if (blockIdx.x < (unsigned)kSumBlocksW) {
         const uint32_t j = blockIdx.x * kSumThreads + threadIdx.x;
         const uint32_t tile = j / kTrTileSums, row = (j >> 2) & (kBM - 1), col = ((j >> 9) & 31u) * 4 + (j & 3u);
@@ -589,6 +595,9 @@ __global__ void __launch_bounds__(kSumThreads) k_train_update(const __grid_const
             i = kOffW2 + ((tile >> 1) * kBM + row) * kHid + (tile & 1) * kTrN + col;
         else
             i = kOffW1 + ((tile - 4) * kBM + row) * kInPad + col;
+        moments();
+        griddep_wait();
+        griddep_launch_dependents();
         const float* part = a.weight_part + j;
         uint32_t q = 0;
         for (; q + 8 <= splits; q += 8) {  // eight in flight, added as a tree
@@ -600,7 +609,14 @@ __global__ void __launch_bounds__(kSumThreads) k_train_update(const __grid_const
         for (; q < splits; ++q) sum += part[(size_t)q * kParams];
     } else {
         const uint32_t b = (blockIdx.x - kSumBlocksW) * (kSumThreads / 32) + (threadIdx.x >> 5);
-        if (b >= (uint32_t)kTrRowSums) return;
+        if (b >= (uint32_t)kTrRowSums) {
+            griddep_wait();
+            return;
+        }
+        i = b < (uint32_t)kHid ? kOffB1 + b : (b < 2u * kHid ? kOffB2 + b - kHid : kOffB3 + b - 2 * kHid);
+        if (b < kTrRowSums - 1) moments();
+        griddep_wait();
+        griddep_launch_dependents();
         const uint32_t tiles = a.B / kBM;
         for (uint32_t q = threadIdx.x & 31; q < tiles; q += 32) sum += a.row_part[(size_t)q * kTrRowSums + b];
 #pragma unroll
@@ -610,16 +626,15 @@ __global__ void __launch_bounds__(kSumThreads) k_train_update(const __grid_const
             if (owner) *a.loss_sum = sum;
             return;
         }
-        i = b < (uint32_t)kHid ? kOffB1 + b : (b < 2u * kHid ? kOffB2 + b - kHid : kOffB3 + b - 2 * kHid);
     }
     if (!owner) return;
     const float gi = sum;
     if constexpr (ADAM) {
-        const float mi = o.b1 * o.m[i] + (1.0f - o.b1) * gi;
-        const float vi = o.b2 * o.v[i] + (1.0f - o.b2) * gi * gi;
+        const float mi = o.b1 * m0 + (1.0f - o.b1) * gi;
+        const float vi = o.b2 * v0 + (1.0f - o.b2) * gi * gi;
         o.m[i] = mi;
         o.v[i] = vi;
-        const float pi = o.p[i] - o.lr * (mi / o.bc1) / (sqrtf(vi / o.bc2) + o.eps);
+        const float pi = p0 - o.lr * (mi / o.bc1) / (sqrtf(vi / o.bc2) + o.eps);
         o.p[i] = pi;
         put_bf16(i, pi, o.w);
     } else {
