@@ -1017,30 +1017,38 @@ marl_status marl_diffuse_device(float* field_dev, float* scratch_dev, const uint
     CellConsts ck;
     derive_consts(*sim, &fk, &ck);
     ResidentPlan rp;
-    const bool resident = resident_plan(g, substeps, sms, &rp);
-    // Workspace: the error word, then the resident kernel's mailboxes or the
-    // padded mask where the caller's rows cannot be read in place.
+    bool resident = resident_plan(g, substeps, sms, &rp);
+    // Workspace: the error word, the resident kernel's mailboxes, the padded mask
+    // where the caller's rows cannot be read in place.
     constexpr size_t head = 256;
     const size_t mail = resident ? resident_mail_bytes(rp) : 0;
-    const bool in_place = resident || mask_in_place(occ_dev, g);
+    const bool in_place = mask_in_place(occ_dev, g);
     uint8_t* work = nullptr;
     CK(work_alloc(&work, head + mail + (in_place ? 0 : (size_t)gz * gy * mask_pitch(gx)), dev, s));
     uint32_t* err = reinterpret_cast<uint32_t*>(work);
     cudaError_t e = cudaMemsetAsync(work, 0, resident ? head + mail : 4, s);
-    const uint8_t* mask = occ_dev;
-    if (!in_place) {
-        mask = work + head;
-        if (e == cudaSuccess) e = launch_repack_mask(occ_dev, work + head, g, s);
-    }
     auto bail = [&](marl_status st) {
         cudaFreeAsync(work, s);
         return st;
     };
-    if (e != cudaSuccess) return bail(cuda_fail(e, "occupancy mask"));
-    if (resident) {
+    if (resident && e == cudaSuccess) {
         e = launch_diffuse_resident(rp, field_dev, occ_dev, gx, g, fk, (int)substeps, 0, nullptr, work + head, 0, err,
                                     s);
-    } else {
+        if (e == cudaErrorCooperativeLaunchTooLarge) {  // a stream that does not have the whole device
+            cudaGetLastError();
+            e = cudaSuccess;
+            resident = false;
+        }
+    }
+    if (e != cudaSuccess) return bail(cuda_fail(e, "diffusion substeps"));
+    if (!resident) {
+        const uint8_t* mask = occ_dev;
+        if (!in_place) {
+            uint8_t* const rows = work + head + mail;
+            mask = rows;
+            if ((e = launch_repack_mask(occ_dev, rows, g, s)) != cudaSuccess)
+                return bail(cuda_fail(e, "occupancy mask"));
+        }
         DiffusionPlan plan;
         int tile, zc;
         default_diffusion_tile(&g, 1, sms, &tile, &zc);

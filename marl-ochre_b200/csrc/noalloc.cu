@@ -96,13 +96,20 @@ extern "C" marl_status marl_diffuse_device_noalloc(float* field_dev, const uint8
     cudaError_t e = cudaMemsetAsync(err, 0, 4, s);
     if (e != cudaSuccess) return cuda_fail(e, "clear error word");
     ResidentPlan rp;
-    if (resident_plan(g, substeps, sms, &rp) && resident_mail_bytes(rp) <= kNoAllocFieldBytes) {
+    bool resident = resident_plan(g, substeps, sms, &rp) && resident_mail_bytes(rp) <= kNoAllocFieldBytes;
+    if (resident) {
         // The kernel's mailboxes in place of the ping-pong copy, which it has no use for.
         if ((e = cudaMemsetAsync(scratch, 0, resident_mail_bytes(rp), s)) == cudaSuccess)
             e = launch_diffuse_resident(rp, field_dev, occupancy_dev, gx, g, fk, (int)substeps, 0, nullptr, scratch, 0,
                                         err, s);
+        if (e == cudaErrorCooperativeLaunchTooLarge) {  // a stream that does not have the whole device
+            cudaGetLastError();
+            e = cudaSuccess;
+            resident = false;
+        }
         if (e != cudaSuccess) return cuda_fail(e, "diffusion substeps");
-    } else {
+    }
+    if (!resident) {
         const bool in_place = mask_in_place(occupancy_dev, g);
         if (!in_place && (e = launch_repack_mask(occupancy_dev, mask, g, s)) != cudaSuccess)
             return cuda_fail(e, "repack occupancy");
