@@ -630,8 +630,9 @@ __global__ void __launch_bounds__(kSumThreads) k_train_update(const __grid_const
     if (!owner) return;
     const float gi = sum;
     if constexpr (ADAM) {
-        const float mi = o.b1 * m0 + (1.0f - o.b1) * gi;
-        const float vi = o.b2 * v0 + (1.0f - o.b2) * gi * gi;
+        // Which product is fused is written out, as in gelu_and_grad().
+        const float mi = __fmaf_rn(1.0f - o.b1, gi, __fmul_rn(o.b1, m0));
+        const float vi = __fmaf_rn(__fmul_rn(1.0f - o.b2, gi), gi, __fmul_rn(o.b2, v0));
         o.m[i] = mi;
         o.v[i] = vi;
         const float pi = p0 - o.lr * (mi / o.bc1) / (sqrtf(vi / o.bc2) + o.eps);

@@ -105,12 +105,19 @@ __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&r)[16
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
-// gelu(z) in the tanh form, and its derivative from the same tanh.
+// gelu(z) = z/2 (1 + t) in the tanh form, t = tanh(c (z + a z^3)), and its
+// derivative (1 + t)/2 + z/2 (1 - t^2) c (1 + 3 a z^2) from the same tanh.  Every
+// rounding is written out: this file is compiled with contraction on, and a product
+// fused otherwise moves h or dz by an ulp, which turns a BF16 rounding here and there
+// and with it single parameters of a run by 1e-3.
 __device__ __forceinline__ float gelu_and_grad(float z, float& grad) {
-    const float u = 0.7978845608028654f * (z + 0.044715f * z * z * z);
-    const float t = tanhf(u);
-    grad = 0.5f * (1.0f + t) + 0.5f * z * (1.0f - t * t) * 0.7978845608028654f * (1.0f + 3.0f * 0.044715f * z * z);
-    return 0.5f * z * (1.0f + t);
+    const float c = 0.7978845608028654f, a = 0.044715f;
+    const float u = __fmul_rn(c, __fmaf_rn(__fmul_rn(__fmul_rn(a, z), z), z, z));
+    const float t = tanhf(u), s = __fadd_rn(1.0f, t), hz = __fmul_rn(0.5f, z);
+    const float w = __fmul_rn(__fmul_rn(hz, __fmaf_rn(-t, t, 1.0f)), c);
+    const float q = __fmaf_rn(__fmul_rn(3.0f * a, z), z, 1.0f);
+    grad = __fmaf_rn(0.5f, s, __fmul_rn(w, q));
+    return __fmul_rn(hz, s);
 }
 // Inference form: the hardware tanh approximation (MUFU), max relative error
 // about 2^-11, below the BF16 rounding the activation goes through next.  Two
