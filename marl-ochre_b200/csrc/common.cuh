@@ -233,9 +233,18 @@ __device__ __forceinline__ void fence_acquire_gpu() { asm volatile("fence.acq_re
 // that the previous kernel reads or writes before griddep_wait() returns,
 // which is when the previous kernel has completed and its writes are
 // visible.  Without such a predecessor both are no-ops.
+//
+// What a kernel before the previous one wrote may be read earlier on two
+// conditions: in every kernel after that writer and before the reader all blocks
+// call griddep_wait() before griddep_launch_dependents() (so that the writer has
+// completed, its writes performed, before the reader can start), and the reader
+// calls reads_before_wait() first (so that no read is served by an older line of
+// L1).  A kernel in between that triggers ahead of its wait, or has none, breaks
+// the first one.
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void griddep_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+__device__ __forceinline__ void reads_before_wait() { fence_acquire_gpu(); }
 
 }  // namespace marl

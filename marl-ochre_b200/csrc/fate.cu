@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kResolveThreads) k_fate_resolve(const FateRun*
 // cell and a moved cell keeps its own voxel, so the two never meet.
 __global__ void __launch_bounds__(256) k_fate_moves(const FateRun* __restrict__ runs) {
     griddep_wait();
-    griddep_launch_dependents();  // after the wait: k_fate_births reads k_fate_resolve's results before its own
+    griddep_launch_dependents();  // after the wait: k_fate_births relies on it (reads_before_wait)
     const FateRun& R = runs[blockIdx.y];
     const Grid g = R.g;
     const uint32_t ndeath = R.f.fs->ndeath;
@@ -405,6 +405,7 @@ __global__ void __launch_bounds__(256) k_fate_moves(const FateRun* __restrict__ 
 __global__ void __launch_bounds__(32 * kFateBirthWarps) k_fate_births(const FateRun* __restrict__ runs,
                                                                       const __grid_constant__ marl_sim_params sim) {
     __shared__ __align__(16) marl_cell rec[kFateBirthWarps];
+    reads_before_wait();  // what k_fate_resolve wrote
     const FateRun& R = runs[blockIdx.y];
     const FateScalars* fs = R.f.fs;
     const uint32_t ndiv = fs->ndiv, n1 = fs->n1;

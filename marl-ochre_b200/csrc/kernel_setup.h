@@ -52,7 +52,7 @@ cudaError_t set_smem_once(std::atomic<int>* slots, K kernel, int bytes) {
 // Launch with programmatic stream serialization: the kernel may be scheduled
 // while the previous kernel of the stream drains, so it must call
 // griddep_wait (common.cuh) before it touches global memory that an earlier
-// launch writes or reads.
+// launch writes or reads; common.cuh names the one exception.
 template <class... KArgs, class... Args>
 cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
                              Args&&... args) {

@@ -582,7 +582,9 @@ __global__ void __launch_bounds__(kSumThreads) k_train_update(const __grid_const
     bool owner = true;
     float sum = 0.0f, m0 = 0.0f, v0 = 0.0f, p0 = 0.0f;
     // Read ahead of the wait: the step before, which wrote them, was over before this
-    // step's row kernel went past its own.
+    // step's row kernel went past its own.  After the wait a step takes 31.4 us at a
+    // batch of 8192 instead of 30.9.
+    if constexpr (ADAM) reads_before_wait();
     auto moments = [&]() {
         if constexpr (ADAM) m0 = __ldcg(o.m + i), v0 = __ldcg(o.v + i), p0 = __ldcg(o.p + i);
     };
