@@ -772,6 +772,8 @@ __device__ __forceinline__ void quad_loop(QuadCell* cells, const CellConsts& c, 
         uint32_t base = 0;
         if (more && free_lanes && lane == 0) base = atomicAdd(ticket, (uint32_t)__popc(free_lanes) >> 2);
         if (run) {  // an update publishes its cell itself
+            // Passes each lane's acquires on to the lanes that gather: a vote orders no memory.
+            __syncwarp();
             const bool updated = quad_update(v, c, C, p, ready);
             if (__any_sync(FULL, !updated)) {
                 if (!updated && p == 0) quad_serial(v.all(), c, C);
