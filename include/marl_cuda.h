@@ -345,7 +345,11 @@ marl_status marl_diffuse_tick_with_cells(marl_ctx* ctx, float* field, const uint
  * Field::scratch, crates/marl-field/src/field.rs:18-20); occupancy_dev is
  * one byte per voxel.  The work is ordered on `cuda_stream` (NULL = legacy
  * default stream); the call synchronizes that stream before returning so that
- * device-side errors are reported. */
+ * device-side errors are reported.  Its workspace (an error word, a padded
+ * occupancy mask, the small grids' exchange buffers) comes from a memory pool
+ * of the library's own, which from the first call on keeps up to 32 MiB of the
+ * device's memory until the process ends or the device is reset;
+ * marl_diffuse_device_noalloc keeps none. */
 marl_status marl_diffuse_device(float* field_dev, float* scratch_dev, const uint8_t* occupancy_dev,
                                 int32_t gx, int32_t gy, int32_t gz, const marl_sim_params* sim,
                                 uint32_t substeps, void* cuda_stream);

@@ -73,33 +73,59 @@ marl_status check_device(int* dev, int* sms) {
 // memory back at every synchronisation (which each of these calls ends with),
 // so an allocation there cost 0.4 ms a call (up to 17 ms among other calls).
 // This pool keeps at most kWorkKeep bytes per device (a pool grows by 32 MiB,
-// so less would keep nothing) and returns what is beyond that at the next
-// synchronisation: 2 us a call.  Pools are safe with several host threads and
-// streams.
+// so less would keep nothing) until the context ends, and returns what is beyond
+// that at the next synchronisation: 2 us a call.  Pools are safe with several
+// host threads and streams.
 constexpr uint64_t kWorkKeep = 32u << 20;
 
-static cudaError_t work_alloc(uint8_t** p, size_t bytes, int dev, cudaStream_t s) {
+// The current context's id, which no later context gets again (a handle may be).
+static bool context_id(unsigned long long* id) {
+    typedef CUresult (*GetId)(CUcontext, unsigned long long*);
+    static const GetId fn = [] {
+        cudaDriverEntryPointQueryResult q;
+        void* p = nullptr;
+        const bool found = cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess &&
+                           q == cudaDriverEntryPointSuccess;
+        return found ? reinterpret_cast<GetId>(p) : nullptr;
+    }();
+    if (!fn) return false;
+    if (fn(nullptr, id) == CUDA_SUCCESS) return true;
+    // No runtime call has made the device's context this thread's yet.
+    return cudaFree(nullptr) == cudaSuccess && fn(nullptr, id) == CUDA_SUCCESS;
+}
+
+// The pool of device `dev` in the current context; null where there is none.
+static cudaMemPool_t work_pool(int dev) {
+    struct Slot {
+        unsigned long long context = 0;
+        cudaMemPool_t pool = nullptr;  // null with a context: refused there once, not tried again
+    };
     static std::mutex lock;
-    static cudaMemPool_t pools[kSetupDevices] = {};
-    if (dev >= 0 && dev < kSetupDevices) {
-        cudaMemPool_t pool = nullptr;
-        {
-            std::lock_guard<std::mutex> hold(lock);
-            if (!pools[dev]) {
-                cudaMemPoolProps props = {};
-                props.allocType = cudaMemAllocationTypePinned;
-                props.location.type = cudaMemLocationTypeDevice;
-                props.location.id = dev;
-                uint64_t keep = kWorkKeep;
-                if (cudaMemPoolCreate(&pool, &props) == cudaSuccess &&
-                    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
-                    pools[dev] = pool;
-            }
-            pool = pools[dev];
-        }
-        if (pool && cudaMallocFromPoolAsync((void**)p, bytes, pool, s) == cudaSuccess) return cudaSuccess;
-        cudaGetLastError();
+    static Slot slots[kSetupDevices];
+    unsigned long long context = 0;
+    if (dev < 0 || dev >= kSetupDevices || !context_id(&context)) return nullptr;
+    std::lock_guard<std::mutex> hold(lock);
+    Slot& s = slots[dev];
+    if (s.context == context) return s.pool;
+    s = Slot{context, nullptr};  // a pool of an earlier context ended with it (a device reset)
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    uint64_t keep = kWorkKeep;
+    if (cudaMemPoolCreate(&s.pool, &props) != cudaSuccess)
+        s.pool = nullptr;
+    else if (cudaMemPoolSetAttribute(s.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaMemPoolDestroy(s.pool);
+        s.pool = nullptr;
     }
+    return s.pool;
+}
+
+static cudaError_t work_alloc(uint8_t** p, size_t bytes, int dev, cudaStream_t s) {
+    if (cudaMemPool_t pool = work_pool(dev))
+        if (cudaMallocFromPoolAsync((void**)p, bytes, pool, s) == cudaSuccess) return cudaSuccess;
+    cudaGetLastError();
     return cudaMallocAsync((void**)p, bytes, s);
 }
 
