@@ -1058,8 +1058,7 @@ marl_status marl_diffuse_device(float* field_dev, float* scratch_dev, const uint
         return st;
     };
     if (resident && e == cudaSuccess) {
-        e = launch_diffuse_resident(rp, field_dev, occ_dev, gx, g, fk, (int)substeps, 0, nullptr, work + head, 0, err,
-                                    s);
+        e = launch_diffuse_resident(rp, field_dev, occ_dev, gx, g, fk, (int)substeps, work + head, err, s);
         if (e == cudaErrorCooperativeLaunchTooLarge) {  // a stream that does not have the whole device
             cudaGetLastError();
             e = cudaSuccess;

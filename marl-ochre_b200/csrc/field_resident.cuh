@@ -53,10 +53,8 @@ struct ResidentArgs {
     Grid g;
     ResidentPlan p;
     FieldConsts k;
-    int substeps, apply_sources;
-    float* c4_out;          // species 4 of the result, compact (nullable)
-    uint4* mail;            // [2][brick][resident_halo][4]; no word holds a tag above `base`
-    uint32_t base;          // substep s sends tag base + s + 1
+    int substeps;
+    uint4* mail;            // [2][brick][resident_halo][4], zeroed; substep s sends tag s + 1
     uint32_t* err;
 };
 
@@ -151,11 +149,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k_diffuse_resident(const __gri
                 __ldcg(reinterpret_cast<const float4*>(a.field + (((size_t)z * g.Y + y) * g.X + x) * 12) + q);
     }
     __syncthreads();
-    if (a.apply_sources)
-        for (int i = tid; i < full; i += kResThreads) {
-            const int lz = i / slab - 1, z = z0 + lz;
-            if (lz <= ez && (z == 0 || z == g.Z - 1)) source_voxel(copy0 + (size_t)i * 12, z, g.Z, a.k);
-        }
 
     // The brick's voxels: the surface that a neighbour reads from the front of
     // the list, the inside from its back; the halo voxels that are read.
@@ -213,7 +206,7 @@ __global__ void __launch_bounds__(kResThreads, 1) k_diffuse_resident(const __gri
         const float* const from = s & 1 ? copy1 : copy0;
         float* const to = s & 1 ? copy0 : copy1;
         uint4* const mail = a.mail + (s & 1 ? mail_set : 0);
-        const uint32_t tag = a.base + (uint32_t)s + 1;
+        const uint32_t tag = (uint32_t)s + 1;
         const bool final_step = s == a.substeps - 1;
         auto update = [&](uint32_t i, bool send) {
             const uint32_t word = list[i], at = word & 0xFFFFu;
@@ -281,7 +274,6 @@ __global__ void __launch_bounds__(kResThreads, 1) k_diffuse_resident(const __gri
             result + (size_t)((lz + 1) * slab + (ly + 1) * row + lx + 1) * 12)[q];
         const size_t at = ((size_t)(z0 + lz) * g.Y + y0 + ly) * g.X + x0 + lx;
         __stcg(reinterpret_cast<float4*>(a.field + at * 12) + q, val);
-        if (q == 1 && a.c4_out) a.c4_out[at] = val.x;
     }
 }
 
@@ -320,12 +312,11 @@ bool resident_plan(const Grid& g, uint32_t substeps, int num_sms, ResidentPlan* 
 }
 
 cudaError_t launch_diffuse_resident(const ResidentPlan& plan, float* field, const uint8_t* mask, int pitch, const Grid& g,
-                                    const FieldConsts& k, int substeps, int apply_sources, float* c4_out, void* mail,
-                                    uint32_t base, uint32_t* err, cudaStream_t s) {
+                                    const FieldConsts& k, int substeps, void* mail, uint32_t* err, cudaStream_t s) {
     static std::atomic<int> setup[kSetupDevices];
     cudaError_t e = set_smem_once(setup, k_diffuse_resident, kResSmemMax);
     if (e != cudaSuccess) return e;
-    ResidentArgs a{field, mask, pitch, g, plan, k, substeps, apply_sources, c4_out, (uint4*)mail, base, err};
+    ResidentArgs a{field, mask, pitch, g, plan, k, substeps, (uint4*)mail, err};
     void* args[] = {&a};
     return cudaLaunchCooperativeKernel((const void*)k_diffuse_resident, dim3(plan.nx * plan.ny * plan.nz),
                                        dim3(kResThreads), args, plan.smem, s);

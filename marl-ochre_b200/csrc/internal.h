@@ -36,12 +36,10 @@ struct ResidentPlan {
 // False where the tiles are faster or the grid does not fit.
 bool resident_plan(const Grid& g, uint32_t substeps, int num_sms, ResidentPlan* plan);
 size_t resident_mail_bytes(const ResidentPlan& p);
-// Two substeps or more on `field` in place.  mail: resident_mail_bytes, 16-byte
-// aligned, in which no 32-bit word at 12 mod 16 lies in base + 1 .. base +
-// substeps (zeroed with base 0, or used before with smaller tags only).
+// Two substeps or more on `field` in place.  mail: resident_mail_bytes, zeroed,
+// 16-byte aligned.
 cudaError_t launch_diffuse_resident(const ResidentPlan& plan, float* field, const uint8_t* mask, int pitch, const Grid& g,
-                                    const FieldConsts& k, int substeps, int apply_sources, float* c4_out, void* mail,
-                                    uint32_t base, uint32_t* err, cudaStream_t s);
+                                    const FieldConsts& k, int substeps, void* mail, uint32_t* err, cudaStream_t s);
 // Tile and z-chunk for a launch over n grids (a rule; the autotuner measures).
 void default_diffusion_tile(const Grid* grids, int n, int num_sms, int* tile, int* zc);
 bool plan_diffusion(DiffusionPlan* plan, const float* a, const float* b, const uint8_t* mask, const Grid& g,

@@ -100,8 +100,7 @@ extern "C" marl_status marl_diffuse_device_noalloc(float* field_dev, const uint8
     if (resident) {
         // The kernel's mailboxes in place of the ping-pong copy, which it has no use for.
         if ((e = cudaMemsetAsync(scratch, 0, resident_mail_bytes(rp), s)) == cudaSuccess)
-            e = launch_diffuse_resident(rp, field_dev, occupancy_dev, gx, g, fk, (int)substeps, 0, nullptr, scratch, 0,
-                                        err, s);
+            e = launch_diffuse_resident(rp, field_dev, occupancy_dev, gx, g, fk, (int)substeps, scratch, err, s);
         if (e == cudaErrorCooperativeLaunchTooLarge) {  // a stream that does not have the whole device
             cudaGetLastError();
             e = cudaSuccess;
