@@ -73,28 +73,44 @@ marl_status check_device(int* dev, int* sms) {
 // memory back at every synchronisation (which each of these calls ends with),
 // so an allocation there cost 0.4 ms a call (up to 17 ms among other calls).
 // This pool keeps at most kWorkKeep bytes per device (a pool grows by 32 MiB,
-// so less would keep nothing) until the context ends, and returns what is beyond
-// that at the next synchronisation: 2 us a call.  Pools are safe with several
+// so less would keep nothing) until its primary context ends, and returns what is
+// beyond that at the next synchronisation: 2 us a call.  Pools are safe with several
 // host threads and streams.
 constexpr uint64_t kWorkKeep = 32u << 20;
 
-// The current context's id, which no later context gets again (a handle may be).
-static bool context_id(unsigned long long* id) {
-    typedef CUresult (*GetId)(CUcontext, unsigned long long*);
-    static const GetId fn = [] {
-        cudaDriverEntryPointQueryResult q;
-        void* p = nullptr;
-        const bool found = cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess &&
-                           q == cudaDriverEntryPointSuccess;
-        return found ? reinterpret_cast<GetId>(p) : nullptr;
-    }();
-    if (!fn) return false;
-    if (fn(nullptr, id) == CUDA_SUCCESS) return true;
-    // No runtime call has made the device's context this thread's yet.
-    return cudaFree(nullptr) == cudaSuccess && fn(nullptr, id) == CUDA_SUCCESS;
+template <class F>
+static F driver_fn(const char* name) {
+    cudaDriverEntryPointQueryResult q;
+    void* p = nullptr;
+    const bool found = cudaGetDriverEntryPoint(name, &p, cudaEnableDefault, &q) == cudaSuccess &&
+                       q == cudaDriverEntryPointSuccess;
+    return found ? reinterpret_cast<F>(p) : nullptr;
 }
 
-// The pool of device `dev` in the current context; null where there is none.
+// The id of the current context, which no later context gets again (a handle
+// may be); false where it is not the device's primary one.
+static bool primary_context_id(int dev, unsigned long long known, unsigned long long* id) {
+    static const auto get_id = driver_fn<CUresult (*)(CUcontext, unsigned long long*)>("cuCtxGetId");
+    static const auto get_current = driver_fn<CUresult (*)(CUcontext*)>("cuCtxGetCurrent");
+    static const auto get_state = driver_fn<CUresult (*)(CUdevice, unsigned int*, int*)>("cuDevicePrimaryCtxGetState");
+    static const auto retain = driver_fn<CUresult (*)(CUcontext*, CUdevice)>("cuDevicePrimaryCtxRetain");
+    static const auto release = driver_fn<CUresult (*)(CUdevice)>("cuDevicePrimaryCtxRelease");
+    if (!get_id || !get_current || !get_state || !retain || !release) return false;
+    if (get_id(nullptr, id) != CUDA_SUCCESS)  // no runtime call has made a context this thread's yet
+        if (cudaFree(nullptr) != cudaSuccess || get_id(nullptr, id) != CUDA_SUCCESS) return false;
+    if (*id == known) return true;
+    CUcontext current = nullptr, primary = nullptr;
+    unsigned int flags;
+    int active = 0;
+    if (get_current(&current) != CUDA_SUCCESS || get_state((CUdevice)dev, &flags, &active) != CUDA_SUCCESS || !active ||
+        retain(&primary, (CUdevice)dev) != CUDA_SUCCESS)
+        return false;
+    release((CUdevice)dev);
+    return current == primary;
+}
+
+// The pool of device `dev`; null where there is none, or in a context other
+// than the primary one (the device's own pool serves there).
 static cudaMemPool_t work_pool(int dev) {
     struct Slot {
         unsigned long long context = 0;
@@ -102,10 +118,11 @@ static cudaMemPool_t work_pool(int dev) {
     };
     static std::mutex lock;
     static Slot slots[kSetupDevices];
-    unsigned long long context = 0;
-    if (dev < 0 || dev >= kSetupDevices || !context_id(&context)) return nullptr;
+    if (dev < 0 || dev >= kSetupDevices) return nullptr;
     std::lock_guard<std::mutex> hold(lock);
     Slot& s = slots[dev];
+    unsigned long long context = 0;
+    if (!primary_context_id(dev, s.context, &context)) return nullptr;
     if (s.context == context) return s.pool;
     s = Slot{context, nullptr};  // a pool of an earlier context ended with it (a device reset)
     cudaMemPoolProps props = {};
