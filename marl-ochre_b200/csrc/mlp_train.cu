@@ -165,6 +165,10 @@ __device__ __forceinline__ void image_load(uint32_t dst, const void* src, uint32
                  "l"(src), "r"(bytes), "r"(smem_u32(bar))
                  : "memory");
 }
+// After an expired wait: waits (bounded) for the phase `parity` of a barrier that
+// image_load()s arrive on, so that no copy lands in shared memory that another block
+// may hold by then.
+__device__ __forceinline__ void image_loads_drain(uint64_t* bar, uint32_t parity) { mbar_wait_bounded(bar, parity); }
 // Generic writes (either block's shared memory) before asynchronous reads.
 __device__ __forceinline__ void fence_proxy_async_all() { asm volatile("fence.proxy.async;" ::: "memory"); }
 
@@ -418,6 +422,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kRowThreads, 1)
     if (tid < kTrN) part[n0 + tid] = (s_col[1][0][tid] + s_col[1][1][tid]) + (s_col[1][2][tid] + s_col[1][3][tid]);
     store_half(a.dz1, P);
     if (tid == 0) image_stores_done();
+    if (warp == kRowThreads / 32 - 1 && lane < 4) image_loads_drain(&w_bar[lane], 0);  // landed long ago, or a wait expired
     tr_teardown<kRowTmem>(t.tmem);
 }
 
@@ -489,6 +494,10 @@ __global__ void __launch_bounds__(kTrThreads) k_train_weights(const __grid_const
                 load(next);
             }
         }
+        if (!ok)
+#pragma unroll 1
+            for (int i = max(0, n - kTrStages); i < n; ++i)
+                image_loads_drain(&bars[i & (kTrStages - 1)], (i / kTrStages) & 1);
         s_ok = ok;
         umma_commit(&bars[2 * kTrStages]);
     }
