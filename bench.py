@@ -9,7 +9,7 @@ then the change list to the host, fate/division/mutation on the host, and the
 edit list back.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl ours|reference]
-    python bench.py --case {diffusion,cells,light,mlp,engine} [...]   (one kernel, for ncu)
+    python bench.py --case {diffusion,cells,light,mlp,engine,train,small} [...]   (one kernel, for ncu)
 
 Printed (rank 0, one JSON line):
   value       ticks/s with all state resident in HBM: K ticks / summed device
@@ -645,6 +645,29 @@ def case_mlp(marl, rows: int, reps: int, rng: np.random.Generator) -> int:
     return 0
 
 
+def case_train(marl, steps, rng) -> int:
+    rows = np.zeros((20_000, 112), np.float32)
+    rows[:, :109] = rng.random((20_000, 109), dtype=np.float32)
+    s = marl.Surrogate(max_pairs=len(rows), batch=8192, seed=1)
+    s.upload_pairs(rows)
+    s.prepare(len(rows))
+    loss = s.train(steps)
+    print(f"train ok: steps={steps} batch=8192 loss={loss[-1]:.4f}")
+    return 0
+
+
+def case_small(marl, dims, substeps, reps, rng) -> int:
+    import torch
+
+    X, Y, Z = dims
+    field = torch.from_numpy(rng.random((Z, Y, X, 12), dtype=np.float32)).cuda()
+    scratch, occ = torch.empty_like(field), torch.zeros((Z, Y, X), dtype=torch.uint8, device="cuda")
+    for _ in range(reps):
+        marl.diffuse_device(field.data_ptr(), scratch.data_ptr(), occ.data_ptr(), dims, marl.default_params(), substeps)
+    print(f"small ok: dims={dims} substeps={substeps} calls={reps}")
+    return 0
+
+
 def run_case(args) -> int:
     import marl_cuda as marl
 
@@ -653,6 +676,10 @@ def run_case(args) -> int:
     rng = np.random.default_rng(1)
     if args.case == "mlp":
         return case_mlp(marl, args.rows, args.reps, rng)
+    if args.case == "train":
+        return case_train(marl, args.reps, rng)
+    if args.case == "small":
+        return case_small(marl, dims, args.substeps, args.reps, rng)
     if args.case == "engine":
         e = marl.Engine(dims, marl.default_params(), rng_seed=42, seed_count=30, cell_capacity=1 << 20)
         if args.device_fate:
@@ -701,12 +728,12 @@ def main() -> int:
     ap.add_argument("--no-surrogate", action="store_true", help="skip the learned-surrogate leg")
     ap.add_argument("--no-micro", action="store_true", help="skip the field and cell microbenchmarks")
     ap.add_argument("--no-device-fate", action="store_true", help="skip the device-fate engine leg")
-    ap.add_argument("--case", choices=["diffusion", "cells", "light", "mlp", "engine"],
+    ap.add_argument("--case", choices=["diffusion", "cells", "light", "mlp", "engine", "train", "small"],
                     help="instead of the benchmark, run one kernel on seeded synthetic inputs (for ncu)")
     ap.add_argument("--dims", type=int, nargs=3, default=[128, 128, 64], help="case grid")
-    ap.add_argument("--substeps", type=int, default=8, help="case diffusion: substeps")
+    ap.add_argument("--substeps", type=int, default=8, help="case diffusion/small: substeps")
     ap.add_argument("--cells", type=int, default=90, help="case cells: random cells")
-    ap.add_argument("--reps", type=int, default=4, help="case cells/light/mlp: repetitions")
+    ap.add_argument("--reps", type=int, default=4, help="case cells/light/mlp/small: repetitions; case train: steps")
     ap.add_argument("--rows", type=int, default=300_000, help="case mlp: rows per inference")
     ap.add_argument("--ticks", type=int, default=1000, help="case engine: ticks of the seed-42 default run")
     ap.add_argument("--device-fate", action="store_true", help="case engine: fate on the device")

@@ -24,7 +24,8 @@
 // epilogues take gelu' from the tanh they have already taken, so the backward
 // ones take none.  The batch is never copied: its rows are drawn by the loads that
 // use them.
-// A step takes 32 us at a batch of 8192 (30 at 512, 200 at 65,536).  With X and the
+// In calls of 50 steps a step takes 32 us at a batch of 8192 (30 at 512, 200 at
+// 65,536; in calls of 200 31, 29, 199).  With X and the
 // moments read after the wait for the kernel before it took 34 (31, 201), with weights
 // gathered 16 bytes a thread and a wait of the block pair before each overwrite it
 // took 37 (34, 220), with rows instead of tile images 54 (50, 335), with a kernel
